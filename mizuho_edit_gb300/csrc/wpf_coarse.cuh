@@ -1,0 +1,720 @@
+// wpf_coarse.cuh -- the coarse part of the multigrid cycle in one launch of one
+// thread-block cluster (sm_103a), included by wpf_solver.cu.
+//
+// What bounds it: latency only.  A half-sweep of a 32^3 level is 16k cell
+// updates; as a kernel of its own it took 2.2-2.7 us, nearly all of it launch
+// and ramp, and the levels below 4096 cells ran in one block at 0.6 us a phase
+// (25-33 us a call).  Here the levels live in the shared memory of up to 16 SMs
+// for the whole sub-cycle (W recursion included):
+//   * level l is cut into slabs of planes along one axis (the one that leaves a
+//     CTA the fewest cells), one per CTA, with one halo plane on each side.  A
+//     CTA that updates a cell of its first or last plane stores it into the
+//     neighbour's halo plane as well, with st.async, whose bytes the
+//     neighbour's mbarrier counts: a half-sweep ends when both halos have landed
+//     and the block has met, without a barrier (and its memory fence, 1100
+//     cycles with 16 CTAs) over the cluster.  Two mbarriers per side, used in
+//     turn, keep a neighbour that is a phase ahead apart; it cannot be two
+//     ahead, since its next phase needs our halo.  The slabs of a level are
+//     twice those of the next coarser one, so restriction and prolongation stay
+//     within a CTA;
+//   * each cell's six couplings and right-hand side, scaled by 1/diag, lie in the
+//     order in which threads take the cells of a colour (two 16-byte vectors per
+//     cell), beside tables of the cell's place in x and its parent's: no index
+//     arithmetic and no boundary test in a sweep; the half-sweeps of one visit
+//     keep all of that in registers and read x only.  With a warp or two per
+//     scheduler every instruction of a phase is latency;
+//   * a level of at most coarse_single() cells belongs to CTA 0 alone (block
+//     barriers), the smallest ones to its first 128 threads and its first warp,
+//     whose barriers are cheaper still.  Right-hand side and correction cross
+//     between the slabs and CTA 0 by st.async as well;
+//   * the host writes the cycle down as a list of operations and the kernel is one
+//     loop over it: each kind of phase is there once, small enough to stay in the
+//     instruction cache (with the recursion inlined, phases of a few cells took
+//     300-1000 cycles, mostly instruction fetch);
+//   * what a red-black cycle makes zero or overwrites is not computed: the first
+//     red half-sweep from a zero guess is 1/diag * b; after a black half-sweep
+//     the black cells carry no residual, so a restriction sums red cells only;
+//     the black half-sweep that follows a prolongation overwrites the black
+//     cells, so only red ones are corrected; and a half-sweep that would repeat
+//     the one before it is skipped.
+#pragma once
+
+#include "wpf_internal.cuh"
+
+namespace wpf {
+
+// Threads per CTA.  Measured (us a launch, 256 / 512 / 1024 threads): FP32 with
+// a first level of 40x36x28 44 / 39 / 56, of 28x25x23 54 / 50 / 66; FP64 (whose
+// idle warps' work would be in the way of the others) 32^3 61 / 69 / 81.
+template <typename R>
+__host__ __device__ constexpr int coarse_nt() { return sizeof(R) == 4 ? 512 : 256; }
+constexpr int COARSE_MAXC = 16;           // CTAs in the cluster (16: opt-in size)
+constexpr size_t COARSE_SMEM = 220 * 1024;
+constexpr int COARSE_MAXL = 12;
+
+// Cells of a level that one CTA keeps to itself: where a phase of one SM costs
+// less than one of the cluster (measured, us a launch: FP32, 28x25x23 first, 50
+// with 1024, 62 with 2500; 32^3 first, 56 with 1024, 69 with 300; FP64, 24x20x18
+// first, 158 with 256 or 600, 181 with 128, 176 with 1100).
+template <typename R>
+__host__ __device__ constexpr int coarse_single() { return sizeof(R) == 4 ? 1024 : 256; }
+
+// One level.  Local axes a (rows), b, c (slabs) are a permutation of x, y, z;
+// strides and couplings follow it.  A row holds hx slots of each colour: slot t
+// of row (lp, b) is the t-th cell of that colour, or, in the last place of a
+// short row, an empty one (zero couplings, a pad cell's place).
+struct CoarseLevel {
+    int na, nb, nc, hx, hb, W, PS;   // x: half rows of pitch W, PS elements a plane and colour
+    int NS, XS;                      // slots and x elements of a colour (their strides)
+    int oA, oB, oD, oX, oT, oP;      // arrays (elements; oT, oP in ints)
+    unsigned mhx, mnb, mhb;          // magic reciprocals (q / d = umulhi(q, m))
+    int dist;                        // cut into slabs (else CTA 0 holds it)
+    int shift;                       // levels from the coarsest one that is cut
+    // of this CTA (filled in by it)
+    int c0, cnt, n;                  // its planes, its slots of a colour
+    int lr, rr;                      // CTAs holding the planes below and above (-1: none)
+    int ldelta, rdelta;              // our place in x -> the mirror's place in theirs
+    unsigned lexp[2], rexp[2];       // bytes that arrive per half-sweep of a colour
+};
+template <typename R>
+struct CoarseSrc {
+    long long sa, sb, sc;            // global strides
+    const R *ca, *cb, *cc, *id, *diag;
+};
+// Operations of the cycle.  nt: the threads that take part; level l is a cut one
+// (every CTA takes part) or CTA 0's.
+enum { OP_RUN = 0,       // count half-sweeps from colour col on (first: from a zero guess)
+       OP_RESTRICT,      // residual of l -> right-hand side of l + 1
+       OP_GATHER,        // the same from a cut level to one of CTA 0
+       OP_SCATTER,       // x of CTA 0's level l + 1 to the CTAs of its children
+       OP_PROLONG };     // x of l += x of l + 1
+struct CoarseOp {
+    unsigned char kind, l, arg, nt32;   // arg: count << 2 | first << 1 | col; nt32: threads / 32
+};
+constexpr int COARSE_MAXOP = 480;
+constexpr int COARSE_MAXK = 256;        // planes of the first level of CTA 0 below cut ones
+
+template <typename R>
+struct CoarseArgs {
+    int nlev, C;             // levels held
+    int ncd;                 // planes of the coarsest level that is cut
+    int lx, oE;              // the first level CTA 0 holds below cut ones; a second rhs array of it
+    unsigned gather;         // bytes that reach CTA 0 in OP_GATHER
+    int nop;
+    CoarseOp op[COARSE_MAXOP];
+    CoarseLevel lv[COARSE_MAXL];
+    CoarseSrc<R> src[COARSE_MAXL];
+    const R* b;              // right-hand side and result of the first level (cell (1,1,1))
+    R* x;
+    double* dot;             // b.x of the first level is added here (or null)
+    int* err;                // set when a bounded wait ran out
+};
+
+// A cell's vectors: {a-, a+, b-, b+} and {c-, c+, 1/diag, rhs}, the couplings to
+// its six neighbours and the right-hand side times 1/diag.
+template <typename R>
+struct alignas(16) Quad {
+    R v[4];
+};
+
+__host__ __device__ inline unsigned coarse_magic(unsigned d) {   // exact for q * d < 2^32
+    return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d);
+}
+__device__ __forceinline__ int coarse_div(int q, unsigned m) { return m ? (int)__umulhi((unsigned)q, m) : q; }
+
+// ---- cluster primitives ---------------------------------------------------------
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of CTA r's copy of a shared-memory location
+__device__ __forceinline__ unsigned peer_addr(const void* p, int r) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), o;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
+    return o;
+}
+// store whose bytes are counted by the mbarrier at `bar` (same CTA as a)
+__device__ __forceinline__ void peer_push(unsigned a, float v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a),
+                 "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void peer_push(unsigned a, double v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void halo_bar_init(uint64_t* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
+}
+__device__ __forceinline__ void halo_bar_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void halo_bar_expect(uint64_t* bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ bool halo_bar_wait(uint64_t* bar, unsigned parity) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+    for (int it = 0; it < (1 << 20); ++it) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// The coarsest cut level has the slabs [r ncd / C, (r + 1) ncd / C); each finer one has them doubled.
+__device__ __forceinline__ int slab_begin(const CoarseLevel& L, int ncd, int C, int r) {
+    return r == C ? L.nc : min(L.nc, (r * ncd / C) << L.shift);
+}
+__device__ __forceinline__ int slab_owner(int shift, int ncd, int C, int c) { return (((c >> shift) + 1) * C - 1) / ncd; }
+
+constexpr unsigned CT_ODD = 1u << 20, CT_LEFT = 1u << 21, CT_RIGHT = 1u << 22;
+
+// The part of a level that depends on the CTA.
+template <typename R>
+__device__ inline void coarse_level_init(CoarseLevel& L, int ncd, int C, int rank) {
+    L.c0 = L.dist ? slab_begin(L, ncd, C, rank) : 0;
+    L.cnt = L.dist ? slab_begin(L, ncd, C, rank + 1) - L.c0 : (rank == 0 ? L.nc : 0);
+    L.n = L.hx * L.nb * L.cnt;
+    L.lr = L.dist && rank > 0 ? rank - 1 : -1;       // (no slab is empty: C <= ncd)
+    L.rr = L.dist && rank + 1 < C ? rank + 1 : -1;
+    L.ldelta = L.lr >= 0 ? (L.c0 - slab_begin(L, ncd, C, L.lr)) * L.PS : 0;   // plane 1 -> their last + 1
+    L.rdelta = -L.cnt * L.PS;                                                 // plane cnt -> 0
+    for (int col = 0; col < 2; ++col) {   // cells of colour col in the planes next to ours
+        L.lexp[col] = (unsigned)(((L.na * L.nb + (((col + L.c0) & 1) ^ 1)) >> 1) * sizeof(R));
+        L.rexp[col] = (unsigned)(((L.na * L.nb + (((col + L.c0 + L.cnt + 1) & 1) ^ 1)) >> 1) * sizeof(R));
+    }
+}
+
+// The relaxed value of a cell: its neighbours at xa[0], xa[1] and the other places.
+template <typename R>
+__device__ __forceinline__ R quad_relax(const Quad<R>& a, const Quad<R>& b, const R* xa, const R* xbm, const R* xbp,
+                                        const R* xcm, const R* xcp) {
+    return (b.v[3] + a.v[0] * xa[0] + a.v[1] * xa[1]) +
+           ((a.v[2] * xbm[0] + a.v[3] * xbp[0]) + (b.v[0] * xcm[0] + b.v[1] * xcp[0]));
+}
+
+template <int K>
+struct CoarseInt {
+    static constexpr int value = K;
+};
+
+// Barrier of a CTA's first nt threads.
+__device__ __forceinline__ void coarse_bar(int nt) {
+    if (nt == 32) __syncwarp();
+    else if (nt == 128) asm volatile("bar.sync 1, 128;" ::: "memory");
+    else __syncthreads();
+}
+
+template <typename R>
+__global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant__ CoarseArgs<R> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ CoarseLevel lv[COARSE_MAXL];
+    // halos [side][parity of the exchange]; rhs from the slabs at CTA 0; correction from CTA 0
+    __shared__ uint64_t bars[6];
+    __shared__ CoarseOp ops[COARSE_MAXOP];
+    __shared__ unsigned char owner[COARSE_MAXK][2];   // CTAs of the children of a plane of level lx
+    R* sm = reinterpret_cast<R*>(smem_raw);
+    const int tid = threadIdx.x;
+    constexpr int NT = coarse_nt<R>();
+    const int C = a.C, nlev = a.nlev;
+    const int rank = C > 1 ? (int)cluster_rank() : 0;
+    for (int q = tid; q < nlev * (int)(sizeof(CoarseLevel) / 4); q += NT)
+        reinterpret_cast<int*>(lv)[q] = reinterpret_cast<const int*>(a.lv)[q];
+    for (int q = tid; q < a.nop; q += NT) ops[q] = a.op[q];
+    if (tid == NT - 1) {
+        for (int q = 0; q < 6; ++q) halo_bar_init(&bars[q]);
+        halo_bar_fence();
+    }
+    __syncthreads();
+    if (tid < nlev) coarse_level_init<R>(lv[tid], a.ncd, C, rank);
+    for (int l = 0; l < nlev; ++l) {   // halos and pads of x read as zero
+        const int n = lv[l].XS * 2 * (int)sizeof(R) / 16;
+        uint4* X = reinterpret_cast<uint4*>(sm + lv[l].oX);
+        for (int q = tid; q < n; q += NT) X[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (a.lx) {
+        for (int q = tid; q < 2 * lv[a.lx].NS; q += NT) sm[a.oE + q] = 0;   // (where there is no second part)
+        const CoarseLevel& L = lv[a.lx - 1];
+        for (int q = tid; q < 2 * lv[a.lx].nc; q += NT)
+            owner[q >> 1][q & 1] = (unsigned char)slab_owner(L.shift, a.ncd, C, min(q, L.nc - 1));
+    }
+    __syncthreads();
+    {   // the operators: one index space over the levels (both colours of a row in
+        // turn), UN slots' loads in flight per thread
+        constexpr int UN = 16 / (int)sizeof(R);
+        int l = 0, base = 0;
+        for (int q0 = tid; l < nlev; q0 += UN * NT) {
+            R ld[UN][9];
+            unsigned place[UN], parent[UN];
+            int at[UN], lq[UN];
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {
+                const int q = q0 + u * NT;
+                while (l < nlev && q - base >= 2 * lv[l].n) base += 2 * lv[l++].n;
+                lq[u] = l;
+                if (l >= nlev) continue;
+                const CoarseLevel& L = lv[l];
+                const CoarseSrc<R>& S = a.src[l];
+                const int m = q - base, r2 = coarse_div(m, L.mhx), t = m - r2 * L.hx;
+                const int row = r2 >> 1, col = r2 & 1;
+                const int lp = coarse_div(row, L.mnb), b = row - lp * L.nb, c = L.c0 + lp;
+                const int e = (col + b + c) & 1;                      // i = col + j + k mod 2, j = b + 1, k = c + 1
+                const int i = e ? 2 * t + 1 : 2 * t + 2;
+                const bool empty = i > L.na;
+                at[u] = col * L.NS + row * L.hx + t;
+#pragma unroll
+                for (int v = 0; v < 9; ++v) ld[u][v] = 0;
+                place[u] = (unsigned)(L.PS + 1);                      // a pad of the first own plane
+                if (!empty) {
+                    const long long g = (i - 1) * S.sa + b * S.sb + c * S.sc;
+                    ld[u][0] = S.ca[g - S.sa];
+                    ld[u][1] = S.ca[g];
+                    ld[u][2] = S.cb[g - S.sb];
+                    ld[u][3] = S.cb[g];
+                    ld[u][4] = S.cc[g - S.sc];
+                    ld[u][5] = S.cc[g];
+                    ld[u][6] = S.id[g];
+                    if (l == 0) ld[u][7] = a.b[g];
+                    if (col == 0) ld[u][8] = S.diag[g];
+                    place[u] = (unsigned)((lp + 1) * L.PS + (b + 1) * L.W + (i >> 1)) | (e ? CT_ODD : 0u) |
+                               (lp == 0 && L.lr >= 0 ? CT_LEFT : 0u) | (lp == L.cnt - 1 && L.rr >= 0 ? CT_RIGHT : 0u);
+                }
+                parent[u] = 0;
+                if (l + 1 < nlev) {   // the parent's x (CTA 0's levels are mirrored in every CTA)
+                    const CoarseLevel& Q = lv[l + 1];
+                    const int I = t, J = b >> 1, K = c >> 1;
+                    parent[u] = (unsigned)(Q.oX + (empty ? Q.PS + 1
+                                                         : ((I + J + K + 1) & 1) * Q.XS + (K - Q.c0 + 1) * Q.PS +
+                                                               (J + 1) * Q.W + ((I + 1) >> 1)));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {
+                if (lq[u] >= nlev) continue;
+                const CoarseLevel& L = lv[lq[u]];
+                const R id = ld[u][6];
+                Quad<R> A, B;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) A.v[v] = ld[u][v] * id;
+                B.v[0] = ld[u][4] * id;
+                B.v[1] = ld[u][5] * id;
+                B.v[2] = id;
+                B.v[3] = ld[u][7] * id;
+                reinterpret_cast<Quad<R>*>(sm + L.oA)[at[u]] = A;
+                reinterpret_cast<Quad<R>*>(sm + L.oB)[at[u]] = B;
+                reinterpret_cast<unsigned*>(sm)[L.oT + at[u]] = place[u];
+                if (at[u] < L.NS) {
+                    sm[L.oD + at[u]] = ld[u][8];
+                    reinterpret_cast<unsigned*>(sm)[L.oP + at[u]] = parent[u];
+                }
+            }
+        }
+    }
+    if (C > 1) cluster_sync();   // every slab is in place before a neighbour writes into its halo
+    else __syncthreads();
+    unsigned uses = 0, phase = 0;   // of each mbarrier (one bit each); exchanges so far
+    bool ok = true;
+    // the neighbours' mbarriers by parity of the exchange: we are the plane above
+    // for the CTA below, and the other way round (scalars: arrays indexed at run
+    // time would live in local memory)
+    unsigned bl0 = 0, bl1 = 0, br0 = 0, br1 = 0;
+    if (rank > 0) {
+        bl0 = peer_addr(&bars[2], rank - 1);
+        bl1 = peer_addr(&bars[3], rank - 1);
+    }
+    if (rank + 1 < C) {
+        br0 = peer_addr(&bars[0], rank + 1);
+        br1 = peer_addr(&bars[1], rank + 1);
+    }
+    auto await = [&](int q) {
+        if (tid < 32 && ok) ok = halo_bar_wait(&bars[q], (uses >> q) & 1u);
+        uses ^= 1u << q;
+    };
+    int nt_before = NT;
+    for (int o = 0; o < a.nop; ++o) {
+        const CoarseOp op = ops[o];
+        const CoarseLevel& L = lv[op.l];
+        const int nt = op.nt32 * 32;
+        if (!L.dist && rank != 0) continue;
+        const bool grows = nt > nt_before;
+        nt_before = nt;
+        if (tid >= nt) continue;
+        if (grows) coarse_bar(nt);   // the smaller group's results
+        const unsigned* T = reinterpret_cast<const unsigned*>(sm) + L.oT;
+        const Quad<R>* A = reinterpret_cast<const Quad<R>*>(sm + L.oA);
+        const Quad<R>* B = reinterpret_cast<const Quad<R>*>(sm + L.oB);
+        R* X = sm + L.oX;
+        const int n = L.n, NS = L.NS, XS = L.XS, W = L.W, PS = L.PS;
+        const bool hl = L.lr >= 0, hr = L.rr >= 0, dist = L.dist;
+        // byte addresses of the mirrors of our x[0] in the neighbours' shared
+        // memory, and the bytes that they send us by colour
+        const unsigned xl = hl ? peer_addr(X + L.ldelta, L.lr) : 0u;
+        const unsigned xr = hr ? peer_addr(X, L.rr) + (unsigned)(L.rdelta * (int)sizeof(R)) : 0u;
+        const unsigned el0 = L.lexp[0], el1 = L.lexp[1], er0 = L.rexp[0], er1 = L.rexp[1];
+        // mirror x of a cell at idx from X
+        auto mirror = [&](unsigned d, unsigned idx, R val) {
+            const unsigned at = idx * (unsigned)sizeof(R);
+            if (d & CT_LEFT) peer_push(xl + at, val, phase & 1u ? bl1 : bl0);
+            if (d & CT_RIGHT) peer_push(xr + at, val, phase & 1u ? br1 : br0);
+        };
+        // end of a phase that changed colour col: both halos have landed
+        auto done = [&](int col) {
+            if (!dist) {
+                coarse_bar(nt);
+                return;
+            }
+            const int p = (int)(phase++ & 1u);
+            if (tid == 0) {   // (bytes that have landed already are counted)
+                if (hl) halo_bar_expect(&bars[p], col ? el1 : el0);
+                if (hr) halo_bar_expect(&bars[2 + p], col ? er1 : er0);
+            }
+            if (hl) await(p);
+            if (hr) await(2 + p);
+            __syncthreads();
+        };
+        if (op.kind == OP_RUN) {
+            const int col = op.arg & 1, count = op.arg >> 2;
+            const bool first = op.arg & 2;
+            // K cells of each colour per thread, in registers
+            auto in_registers = [&](auto kc) {
+                constexpr int K = decltype(kc)::value;
+                struct Cell {
+                    Quad<R> a, b;
+                    R* x;
+                    const R *xa, *xbm, *xbp, *xcm, *xcp;
+                    unsigned d, idx;
+                } c0[K], c1[K];
+                auto fetch = [&](Cell& c, int cc, int m) {
+                    const bool on = m < n;
+                    const int at = cc * NS + (on ? m : 0);
+                    c.a = A[at];
+                    c.b = B[at];
+                    const unsigned d = T[at];
+                    const int o = (int)(d & (CT_ODD - 1));
+                    const R* O = X + (cc ^ 1) * XS + o;
+                    c.idx = (unsigned)(cc * XS + o);
+                    c.x = on ? X + c.idx : nullptr;
+                    c.d = on ? d : 0u;
+                    c.xa = O - ((d & CT_ODD) ? 0 : 1);
+                    c.xbm = O - W;
+                    c.xbp = O + W;
+                    c.xcm = O - PS;
+                    c.xcp = O + PS;
+                };
+                auto half = [&](Cell* c, int cc, bool zero) {
+                    R val[K];
+#pragma unroll
+                    for (int q = 0; q < K; ++q) {
+                        // (an idle warp spares the narrow FP64 pipe; in FP32 a branch costs more)
+                        if (sizeof(R) == 8 && !c[q].x) continue;
+                        val[q] = zero ? c[q].b.v[3]
+                                      : quad_relax(c[q].a, c[q].b, c[q].xa, c[q].xbm, c[q].xbp, c[q].xcm, c[q].xcp);
+                    }
+#pragma unroll
+                    for (int q = 0; q < K; ++q) {
+                        if (c[q].x) *c[q].x = val[q];
+                        if (dist) mirror(c[q].d, c[q].idx, val[q]);   // (d is 0 where there is no cell)
+                    }
+                    done(cc);
+                };
+#pragma unroll
+                for (int q = 0; q < K; ++q) {
+                    fetch(c0[q], col, tid + q * NT);
+                    fetch(c1[q], col ^ 1, tid + q * NT);
+                }
+                for (int p = 0; p < count; p += 2) {
+                    half(c0, col, first && p == 0);
+                    if (p + 1 < count) half(c1, col ^ 1, false);
+                }
+            };
+            if (n <= nt) {
+                in_registers(CoarseInt<1>{});
+            } else if (sizeof(R) == 4 && n <= 2 * NT && nt == NT) {   // (FP64: out of registers)
+                in_registers(CoarseInt<sizeof(R) == 4 ? 2 : 1>{});
+            } else {
+                int cc = col;
+                for (int p = 0; p < count; ++p, cc ^= 1) {
+                    const R* Y = X + (cc ^ 1) * XS;
+                    for (int m = tid; m < n; m += nt) {
+                        const unsigned d = T[cc * NS + m], o = d & (CT_ODD - 1);
+                        const Quad<R> qb = B[cc * NS + m];
+                        R val = qb.v[3];
+                        if (!(first && p == 0)) {
+                            const R* O = Y + o;
+                            val = quad_relax(A[cc * NS + m], qb, O - ((d & CT_ODD) ? 0 : 1), O - W, O + W, O - PS, O + PS);
+                        }
+                        X[cc * XS + o] = val;
+                        mirror(d, (unsigned)(cc * XS) + o, val);
+                    }
+                    done(cc);
+                }
+            }
+        } else if (op.kind == OP_RESTRICT || op.kind == OP_GATHER) {
+            // right-hand side of the next level := residual summed over each aggregate
+            // (red cells: the black ones were relaxed last; the red cell of aggregate I
+            // in a row is the row's slot I).  To CTA 0, an aggregate whose second
+            // plane is another CTA's gets that part in a second array.  With x* the
+            // relaxed value of a cell, its residual is diag (x* - x).
+            const CoarseLevel& Q = lv[op.l + 1];
+            const bool gather = op.kind == OP_GATHER;
+            const unsigned to = gather ? peer_addr(sm + Q.oB, 0) : 0u, extra = gather ? peer_addr(sm + a.oE, 0) : 0u;
+            const unsigned bar = gather ? peer_addr(&bars[4], 0) : 0u;
+            const int c0 = L.c0, K0 = c0 >> 1, hx = L.hx, hb = L.hb, nb = L.nb, cnt = L.cnt;
+            const int agg = hx * hb * (((c0 + cnt - 1) >> 1) - K0 + 1);
+            const R* D = sm + L.oD;
+            for (int m = tid; m < agg; m += nt) {
+                const int r = coarse_div(m, L.mhx), I = m - r * hx;
+                const int kk = coarse_div(r, L.mhb), J = r - kk * hb, K = K0 + kk;
+                R s = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int b = 2 * J + (q & 1), lp = 2 * K + (q >> 1) - c0;
+                    if (b >= nb || lp < 0 || lp >= cnt) continue;
+                    const int t = (lp * nb + b) * hx + I;
+                    const unsigned d = T[t], idx = d & (CT_ODD - 1);
+                    const R* O = X + XS + idx;
+                    s += D[t] * (quad_relax(A[t], B[t], O - ((d & CT_ODD) ? 0 : 1), O - W, O + W, O - PS, O + PS) - X[idx]);
+                }
+                const int at = ((I + J + K + 1) & 1) * Q.NS + ((K - Q.c0) * Q.nb + J) * Q.hx + (I >> 1);
+                if (!gather) sm[Q.oB + at * 4 + 3] = s * sm[Q.oB + at * 4 + 2];
+                else if (2 * K < c0) peer_push(extra + (unsigned)at * (unsigned)sizeof(R), s, bar);
+                else peer_push(to + (unsigned)(at * 4 + 3) * (unsigned)sizeof(R), s, bar);
+            }
+            if (gather) {
+                if (rank != 0) continue;
+                if (tid == 0) halo_bar_expect(&bars[4], a.gather);
+                await(4);
+                __syncthreads();
+                for (int m = tid; m < 2 * Q.NS; m += NT) sm[Q.oB + m * 4 + 3] = (sm[Q.oB + m * 4 + 3] + sm[a.oE + m]) * sm[Q.oB + m * 4 + 2];
+            }
+            coarse_bar(nt);
+        } else if (op.kind == OP_SCATTER) {
+            const CoarseLevel& Q = lv[op.l + 1];
+            if (rank == 0) {
+                for (int m = tid; m < 2 * Q.NS; m += NT) {
+                    const int col = m >= Q.NS, t = m - col * Q.NS;
+                    if (t >= Q.n) continue;
+                    const int K = coarse_div(coarse_div(t, Q.mhx), Q.mnb);
+                    const unsigned idx = reinterpret_cast<const unsigned*>(sm)[Q.oT + m] & (CT_ODD - 1);
+                    const R* x = sm + Q.oX + col * Q.XS + idx;
+                    const int f = owner[K][0], g = owner[K][1];
+                    const R v = *x;
+                    if (f) peer_push(peer_addr(x, f), v, peer_addr(&bars[5], f));
+                    if (g != f) peer_push(peer_addr(x, g), v, peer_addr(&bars[5], g));
+                }
+            } else {
+                const int planes = ((L.c0 + L.cnt - 1) >> 1) - (L.c0 >> 1) + 1;
+                if (tid == 0) halo_bar_expect(&bars[5], (unsigned)(planes * 2 * Q.hx * Q.nb * (int)sizeof(R)));
+                await(5);
+                __syncthreads();
+            }
+        } else {   // OP_PROLONG: the live red cells (a dead one stays 0; black ones are relaxed next)
+            const unsigned* P = reinterpret_cast<const unsigned*>(sm) + L.oP;
+            for (int m = tid; m < n; m += nt) {
+                const unsigned d = T[m], idx = d & (CT_ODD - 1);
+                const R add = sm[P[m]], id = B[m].v[2];
+                const R val = id == (R)0 ? (R)0 : X[idx] + add;
+                X[idx] = val;
+                mirror(d, idx, val);
+            }
+            done(0);
+        }
+    }
+    __syncthreads();
+    // the result of the first level
+    {
+        const CoarseLevel& L = lv[0];
+        const CoarseSrc<R>& S = a.src[0];
+        R dot = 0;
+        for (int m = tid; m < 2 * L.n; m += NT) {
+            const int r2 = coarse_div(m, L.mhx), t = m - r2 * L.hx;
+            const int row = r2 >> 1, col = r2 & 1;
+            const int lp = coarse_div(row, L.mnb), b = row - lp * L.nb, c = L.c0 + lp;
+            const int i = ((col + b + c) & 1) ? 2 * t + 1 : 2 * t + 2, s = col * L.NS + row * L.hx + t;
+            if (i > L.na) continue;
+            const unsigned d = reinterpret_cast<const unsigned*>(sm)[L.oT + s];
+            const R val = sm[L.oX + col * L.XS + (int)(d & (CT_ODD - 1))];
+            const long long g = (i - 1) * S.sa + b * S.sb + c * S.sc;
+            a.x[g] = val;
+            if (a.dot) dot += a.b[g] * val;
+        }
+        if (a.dot && (L.dist || rank == 0)) block_add(dot, a.dot);
+    }
+    if (!ok && tid == 0 && a.err) atomicExch(a.err, 1);
+    if (C > 1) cluster_sync();   // no CTA leaves while a neighbour may still store into it
+}
+
+// The cycle's operations: levels 0..nv-1 recurse (those in wmask twice), the
+// others are a V-cycle.  False when the list is too short for them.
+template <typename R>
+bool coarse_ops(CoarseArgs<R>& a, int nv, unsigned wmask, int nu) {
+    a.nop = 0;
+    bool fits = nu <= 16;   // (counts of half-sweeps up to 63)
+    auto nt32 = [&](int l) {
+        const CoarseLevel& L = a.lv[l];
+        const int n = L.hx * L.nb * L.nc;
+        return L.dist || n > 128 ? coarse_nt<R>() / 32 : (n > 32 ? 4 : 1);
+    };
+    auto put = [&](int kind, int l, int arg, int nt) {
+        if (a.nop == COARSE_MAXOP) fits = false;
+        else a.op[a.nop++] = CoarseOp{(unsigned char)kind, (unsigned char)l, (unsigned char)arg, (unsigned char)nt};
+    };
+    auto run = [&](int l, int col, int count, bool first) {
+        put(OP_RUN, l, count << 2 | (first ? 2 : 0) | col, nt32(l));
+    };
+    auto down = [&](int l, bool zero) {   // pre-smoothing and right-hand side of l + 1
+        // (not from zero: the symmetric sweeps before ended with the first half-sweep)
+        run(l, zero ? 0 : 1, zero ? 2 * nu : 2 * nu - 1, zero);
+        put(a.lv[l].dist && !a.lv[l + 1].dist ? OP_GATHER : OP_RESTRICT, l, 0, nt32(l));
+    };
+    auto up = [&](int l) {
+        if (a.lv[l].dist && !a.lv[l + 1].dist) put(OP_SCATTER, l, 0, nt32(l));
+        put(OP_PROLONG, l, 0, nt32(l));
+        run(l, 1, 2 * nu, false);
+    };
+    const int last = a.nlev - 1;
+    int l = 0;
+    unsigned rep = 0;
+    bool descend = true;
+    while (fits) {
+        if (descend) {
+            if (l < last) {
+                down(l, true);
+                ++l;
+                continue;
+            }
+            run(l, 0, 9, true);   // the coarsest: four symmetric pairs from zero (repeats left out)
+            descend = false;
+        } else {
+            up(l);
+            if (l < nv && ((wmask >> l) & 1u) && !((rep >> l) & 1u)) {
+                rep |= 1u << l;
+                down(l, false);
+                ++l;
+                descend = true;
+                continue;
+            }
+            rep &= ~(1u << l);
+        }
+        if (l == 0) break;
+        --l;
+    }
+    return fits;
+}
+
+// Levels l0.. of H, cut along axis `cut`, as the cluster kernel's arguments; the
+// shared memory they take (0: they do not fit).  nv: the first level of the
+// plain V-cycle on CTA 0; wmask: bit l: level l recurses twice.
+template <typename R>
+size_t coarse_args(const Hierarchy<R>& H, int l0, int nv, unsigned wmask, int nu, int maxc, int cut,
+                   CoarseArgs<R>& a) {
+    a.nlev = H.nlev - l0;
+    if (a.nlev < 1 || a.nlev > COARSE_MAXL) return 0;
+    const int ax[3] = {cut == 0 ? 1 : 0, cut == 2 ? 1 : 2, cut};   // rows along x when that is free
+    nv = nv > l0 ? nv - l0 : 0;
+    int ld = -1;   // the coarsest level that is cut
+    for (int l = 0; l < a.nlev; ++l) {
+        const Level<R>& S = H.lv[l0 + l];
+        CoarseLevel& L = a.lv[l];
+        CoarseSrc<R>& G = a.src[l];
+        const int n[3] = {S.g.nx, S.g.ny, S.g.nz};
+        const long long st[3] = {1, S.g.P, S.g.S};
+        const R* cp[3] = {S.cx, S.cy, S.cz};
+        const long long base = S.g.at(1, 1, 1);
+        L = CoarseLevel();
+        L.na = n[ax[0]]; L.nb = n[ax[1]]; L.nc = n[ax[2]];
+        G.sa = st[ax[0]]; G.sb = st[ax[1]]; G.sc = st[ax[2]];
+        G.ca = cp[ax[0]] + base; G.cb = cp[ax[1]] + base; G.cc = cp[ax[2]] + base;
+        G.id = S.idiag + base;
+        G.diag = S.diag + base;
+        const long long cells = (long long)L.na * L.nb * L.nc;
+        if (cells > (1 << 18)) return 0;
+        // (a plane of one cell lacks a colour, and a half-sweep its exchange)
+        L.dist = cells > coarse_single<R>() && l < nv && ld == l - 1 && L.na * L.nb >= 2;
+        if (L.dist) ld = l;
+        if (l == 0) { a.b = S.b + base; a.x = S.x + base; }
+    }
+    a.C = 1;
+    a.ncd = 1;
+    if (ld >= 0) {   // as few CTAs as the same number of planes each allows
+        a.ncd = a.lv[ld].nc;
+        const int per = (a.ncd + maxc - 1) / maxc;
+        a.C = (a.ncd + per - 1) / per;
+    }
+    a.lx = a.oE = 0;
+    long long off = 0;
+    for (int l = 0; l < a.nlev; ++l) {
+        CoarseLevel& L = a.lv[l];
+        L.dist = L.dist && a.C > 1;
+        L.shift = L.dist ? ld - l : 0;
+        int planes = L.nc;
+        if (L.dist && (((a.ncd + a.C - 1) / a.C) << L.shift) < planes) planes = ((a.ncd + a.C - 1) / a.C) << L.shift;
+        L.hx = (L.na + 1) / 2;
+        L.hb = (L.nb + 1) / 2;
+        L.W = L.hx + 1;
+        L.PS = L.W * (L.nb + 2);
+        L.NS = (L.hx * L.nb * planes + 3) & ~3;
+        L.XS = (L.PS * (planes + 2) + 3) & ~3;
+        L.mhx = coarse_magic(L.hx);
+        L.mnb = coarse_magic(L.nb);
+        L.mhb = coarse_magic(L.hb);
+        // two vectors per slot, x, diag per red slot; two tables (ints)
+        const int ints = (int)sizeof(R) / 4;
+        L.oA = (int)off;
+        L.oB = L.oA + 8 * L.NS;
+        L.oX = L.oB + 8 * L.NS;
+        L.oD = L.oX + 2 * L.XS;
+        L.oT = (L.oD + L.NS) * ints;
+        L.oP = L.oT + 2 * L.NS;
+        off = L.oD + L.NS + (3LL * L.NS + ints - 1) / ints;
+        if (l > 0 && a.lv[l - 1].dist && !L.dist) {
+            a.lx = l;
+            a.oE = (int)off;
+            off += 2 * L.NS;
+            // a part of each plane, a second one where a slab ends between its children
+            int parts = L.nc;
+            for (int r = 1; r < a.C; ++r) parts += ((r * a.ncd / a.C) << a.lv[l - 1].shift) & 1;
+            a.gather = (unsigned)(parts * L.na * L.nb * (int)sizeof(R));
+            if (L.nc > COARSE_MAXK) return 0;
+        }
+        off = (off + 3) & ~3LL;
+        if (off * (long long)sizeof(R) > (long long)COARSE_SMEM || L.XS >= (1 << 20)) return 0;
+    }
+    if (!coarse_ops(a, nv, wmask >> l0, nu)) return 0;
+    return (size_t)off * sizeof(R);
+}
+
+// The same along the axis that leaves a CTA the fewest cells of the first level.
+template <typename R>
+size_t coarse_fit(const Hierarchy<R>& H, int l0, int nv, unsigned wmask, int nu, int maxc, CoarseArgs<R>& a) {
+    size_t best = 0;
+    long long cells = 0;
+    CoarseArgs<R> t = {};
+    for (int cut = 2; cut >= 0; --cut) {
+        const size_t sm = coarse_args(H, l0, nv, wmask, nu, maxc, cut, t);
+        if (!sm) continue;
+        const CoarseLevel& L = t.lv[0];
+        long long planes = L.dist ? (long long)((t.ncd + t.C - 1) / t.C) << L.shift : L.nc;
+        if (planes > L.nc) planes = L.nc;
+        const long long n = planes * L.na * L.nb;
+        if (best && n >= cells) continue;
+        best = sm;
+        cells = n;
+        a = t;
+    }
+    return best;
+}
+
+}  // namespace wpf

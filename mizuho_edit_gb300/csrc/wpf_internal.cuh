@@ -352,7 +352,7 @@ enum KClass {
     KC_VEC,           // PCG vector updates / dots / correction
     KC_FUSED,         // fused velocity + phase + concentration + Euler + halo
     KC_OTHER,         // halo, Dirichlet, reductions
-    KC_BOTTOM,        // single-block bottom cycle of the hierarchy
+    KC_BOTTOM,        // the coarse levels' sub-cycle (one cluster launch)
     KC_COUNT
 };
 // Record a start event for class c (if timed); returns the slot or -1.

@@ -36,7 +36,8 @@
 // so every block produces exactly the two-kernel red-black result; the sweep
 // reads x from one buffer and writes the other, so no block can see another
 // block's new values.  Mid-size levels use in-place two-kernel half-sweeps and
-// the levels of at most 4096 cells run their whole sub-cycle in one block.
+// the levels that fit the shared memory of a thread-block cluster run their
+// whole sub-cycle in one launch (wpf_coarse.cuh).
 #include <cuda.h>   // CUtensorMap (the encoder is fetched at run time)
 #include <math.h>
 
@@ -45,6 +46,7 @@
 #include <stdio.h>
 
 #include "wpf_internal.cuh"
+#include "wpf_coarse.cuh"
 
 namespace wpf {
 
@@ -998,191 +1000,6 @@ __global__ void k_resid_restrict(Grid f, Grid c, const R* __restrict__ cx, const
     bc[c.at(I, J, K)] = s;
 }
 
-// The coarsest levels (at most bottom_cells<R>() cells on the first of them)
-// run their whole sub-cycle in one 1024-thread block, with every array of
-// those levels copied into shared memory in a compact halo-free layout
-// (neighbours outside the grid read as zero; their couplings are zero).
-constexpr int BOTTOM_THREADS = 1024;
-constexpr size_t BOTTOM_SMEM_MAX = 200 * 1024;   // bound on the staged bottom levels
-template <typename R>
-constexpr long long bottom_cells() { return sizeof(R) == 4 ? 4096 : 512; }
-
-template <typename R>
-struct BottomArgs {
-    int l0, nlev, nu;
-    Level<R> lv[MAX_LEVELS];
-};
-
-template <typename R>
-struct BLevel {
-    int nx, ny, nz, n, hx;   // hx = cells of one colour per row, at most
-    // q / d = (q * ceil(2^32 / d)) >> 32, exact for q * d < 2^32 (here q, d < 2^13)
-    unsigned long long mnx, mny, mhx;
-    R *cx, *cy, *cz, *d, *id, *x, *b;
-};
-
-__host__ __device__ inline unsigned long long div_magic(unsigned d) {
-    return ((1ull << 32) + d - 1) / d;
-}
-__device__ __forceinline__ int fdiv(int q, unsigned long long m) {
-    return (int)(((unsigned long long)(unsigned)q * m) >> 32);
-}
-
-template <typename R>
-__device__ __forceinline__ R b_offsum(const BLevel<R>& L, int c, int i, int j, int k) {
-    const int sy = L.nx, sz = L.nx * L.ny;
-    R s = 0;
-    if (i + 1 < L.nx) s += L.cx[c] * L.x[c + 1];
-    if (i > 0) s += L.cx[c - 1] * L.x[c - 1];
-    if (j + 1 < L.ny) s += L.cy[c] * L.x[c + sy];
-    if (j > 0) s += L.cy[c - sy] * L.x[c - sy];
-    if (k + 1 < L.nz) s += L.cz[c] * L.x[c + sz];
-    if (k > 0) s += L.cz[c - sz] * L.x[c - sz];
-    return s;
-}
-
-// colour of a 0-based cell in the 1-based convention of the other kernels
-__device__ __forceinline__ int b_colour(int i, int j, int k) { return (i + j + k + 1) & 1; }
-
-// One colour of Gauss-Seidel on a staged level: thread m takes the m-th cell of
-// that colour (row r = (j,k), t-th of the row).  first: the zero-guess first
-// sweep, which also zeroes the other colour (x = 0 before it).
-template <typename R>
-__device__ __forceinline__ void b_sweep(const BLevel<R> L, int color, bool first = false) {
-    const int nh = L.hx * L.ny * L.nz;
-    for (int m = threadIdx.x; m < nh; m += blockDim.x) {
-        const int r = fdiv(m, L.mhx), t = m - r * L.hx, k = fdiv(r, L.mny), j = r - k * L.ny;
-        const int par = (color + 1 + j + k) & 1;   // b_colour(i, j, k) == color
-        const int i = 2 * t + par;
-        const int c = i + L.nx * r;
-        if (first) {
-            if (i < L.nx) L.x[c] = L.id[c] * L.b[c];
-            const int io = 2 * t + (par ^ 1);
-            if (io < L.nx) L.x[c - i + io] = 0;
-        } else if (i < L.nx) {
-            L.x[c] = L.id[c] * (L.b[c] + b_offsum(L, c, i, j, k));
-        }
-    }
-    __syncthreads();
-}
-
-// b of level l+1 = residual of level l summed over each aggregate.
-template <typename R>
-__device__ __forceinline__ void b_restrict(const BLevel<R> L, const BLevel<R> C) {
-    for (int q = threadIdx.x; q < C.n; q += blockDim.x) {
-        const int rr = fdiv(q, C.mnx), I = q - rr * C.nx, K = fdiv(rr, C.mny), J = rr - K * C.ny;
-        R s = 0;
-        for (int dk = 0; dk < 2; ++dk) {
-            const int k = 2 * K + dk;
-            if (k >= L.nz) break;
-            for (int dj = 0; dj < 2; ++dj) {
-                const int j = 2 * J + dj;
-                if (j >= L.ny) break;
-                for (int di = 0; di < 2; ++di) {
-                    const int i = 2 * I + di;
-                    if (i >= L.nx) break;
-                    const int c = i + L.nx * (j + L.ny * k);
-                    s += L.b[c] - (L.d[c] * L.x[c] - b_offsum(L, c, i, j, k));
-                }
-            }
-        }
-        C.b[q] = s;
-    }
-    __syncthreads();
-}
-
-template <typename R>
-__device__ __forceinline__ void b_prolong(const BLevel<R> L, const BLevel<R> C) {
-    for (int c = threadIdx.x; c < L.n; c += blockDim.x) {
-        const int r = fdiv(c, L.mnx), i = c - r * L.nx, k = fdiv(r, L.mny), j = r - k * L.ny;
-        if (L.id[c] != (R)0) L.x[c] += C.x[(i >> 1) + C.nx * ((j >> 1) + C.ny * (k >> 1))];
-    }
-    __syncthreads();
-}
-
-// V-cycle over the staged levels l0..last, written as two loops (no device
-// recursion, so no call stack): nu symmetric red-black sweeps around each
-// coarse correction.  The coarsest level (at most 2 cells per axis) is one
-// cell in the usual case, solved exactly; otherwise it gets 4 symmetric
-// red-black sweep pairs from zero -- a symmetric operator, like the rest.
-template <typename R>
-__device__ void b_vcycle(const BLevel<R>* lv, int l0, int last, int nu) {
-    for (int l = l0; l < last; ++l) {
-        const BLevel<R> L = lv[l];
-        b_sweep(L, 0, true);
-        b_sweep(L, 1);
-        for (int s = 1; s < nu; ++s) { b_sweep(L, 0); b_sweep(L, 1); }
-        b_restrict(L, lv[l + 1]);
-    }
-    {
-        const BLevel<R> L = lv[last];
-        if (L.n == 1) {
-            if (threadIdx.x == 0) L.x[0] = L.id[0] * L.b[0];
-            __syncthreads();
-        } else {
-            b_sweep(L, 0, true);
-            b_sweep(L, 1);
-            b_sweep(L, 1);
-            b_sweep(L, 0);
-            for (int s = 1; s < 4; ++s) { b_sweep(L, 0); b_sweep(L, 1); b_sweep(L, 1); b_sweep(L, 0); }
-        }
-    }
-    for (int l = last - 1; l >= l0; --l) {
-        const BLevel<R> L = lv[l];
-        b_prolong(L, lv[l + 1]);
-        for (int s = 0; s < nu; ++s) { b_sweep(L, 1); b_sweep(L, 0); }
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(BOTTOM_THREADS) k_bottom(BottomArgs<R> A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* sp = reinterpret_cast<R*>(smem_raw);
-    __shared__ BLevel<R> lv[MAX_LEVELS];
-    if (threadIdx.x == 0) {
-        R* p = sp;
-        for (int l = A.l0; l < A.nlev; ++l) {
-            const Grid& g = A.lv[l].g;
-            BLevel<R>& B = lv[l];
-            B.nx = g.nx; B.ny = g.ny; B.nz = g.nz; B.n = g.nx * g.ny * g.nz;
-            B.hx = (g.nx + 1) / 2;
-            B.mnx = div_magic(g.nx);
-            B.mny = div_magic(g.ny);
-            B.mhx = div_magic(B.hx);
-            R** arrs[7] = {&B.cx, &B.cy, &B.cz, &B.d, &B.id, &B.x, &B.b};
-            for (auto a : arrs) { *a = p; p += B.n; }
-        }
-    }
-    __syncthreads();
-    for (int l = A.l0; l < A.nlev; ++l) {   // stage the operators and the top right-hand side
-        const Level<R>& G = A.lv[l];
-        const BLevel<R> B = lv[l];
-        for (int c = threadIdx.x; c < B.n; c += blockDim.x) {
-            const int r = fdiv(c, B.mnx), i = c - r * B.nx, k = fdiv(r, B.mny), j = r - k * B.ny;
-            const long long n = G.g.at(i + 1, j + 1, k + 1);
-            const R vx = G.cx[n], vy = G.cy[n], vz = G.cz[n], vd = G.diag[n], vi = G.idiag[n];
-            const R vb = l == A.l0 ? G.b[n] : (R)0;
-            B.cx[c] = vx; B.cy[c] = vy; B.cz[c] = vz; B.d[c] = vd; B.id[c] = vi;
-            if (l == A.l0) B.b[c] = vb;
-        }
-    }
-    __syncthreads();
-    b_vcycle(lv, A.l0, A.nlev - 1, A.nu);
-    const Level<R>& G = A.lv[A.l0];
-    const BLevel<R> B = lv[A.l0];
-    for (int c = threadIdx.x; c < B.n; c += blockDim.x) {
-        const int r = fdiv(c, B.mnx), i = c - r * B.nx, k = fdiv(r, B.mny), j = r - k * B.ny;
-        G.x[G.g.at(i + 1, j + 1, k + 1)] = B.x[c];
-    }
-}
-
-template <typename R>
-static size_t bottom_smem(const Hierarchy<R>& H, int l0) {
-    size_t cells = 0;
-    for (int l = l0; l < H.nlev; ++l) cells += (size_t)H.lv[l].g.nx * H.lv[l].g.ny * H.lv[l].g.nz;
-    return cells * 7 * sizeof(R);
-}
-
 // ---- PCG vector kernels (persistent row loops, one atomic per block) -------
 // p_new = z + beta p_old (beta = rz_new/rz_old, 0 when first) formed on the
 // fly for the cell and its six neighbours; q = A' p_new; accumulates p_new.q.
@@ -1457,8 +1274,8 @@ constexpr long long BIG_CELLS = 1LL << 23;   // default: levels swept by the pip
 // a symmetric preconditioner.  Big levels sweep between their two buffers so
 // that the 2*nu sweeps end in the level's output buffer x (the first
 // pre-sweep writes xs, the last post-sweep writes x); mid levels sweep x in
-// place; the levels from the first one with at most bottom_cells<R>() cells
-// run in one k_bottom block.
+// place; the levels that fit a cluster's shared memory run in one k_coarse launch
+// (wpf_coarse.cuh).
 // ---- bulk-tensor maps of the sweep -------------------------------------------------
 EncodeTiledFn tensor_map_encoder() {
     static EncodeTiledFn fn = nullptr;
@@ -1572,19 +1389,73 @@ static void launch_sweep(wpf_handle* h, Hierarchy<R>& H, int l, int cls, bool ze
             g, L.cx, L.cy, L.cz, L.idiag, L.b, in, out, c0, dot, m, err, szc));
 }
 
+// Levels of at most this many cells (FP32 / FP64) run a plain V-cycle.
 template <typename R>
-static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, int lb, int nu, long long big,
+constexpr long long vcycle_cells() { return sizeof(R) == 4 ? 4096 : 512; }
+
+// The levels that k_coarse takes: from the finest one that fits its shared
+// memory (with cells < COARSE_TOP) down.  Per preconditioner cycle, launches on
+// those levels before -> after: 100x90x110 FP32 100 -> 50 us, 64^3 FP64 (L1 down)
+// 230 -> 60 us, 96x80x72 FP64 (L2 down) 300 -> 128 us.
+template <typename R>
+struct CoarsePlan {
+    int l0;
+    size_t smem;
+    CoarseArgs<R> args;
+};
+// (46^3 in FP32 still fits, and a half-sweep over it costs ~0.9 us there against
+// the launch's 2.2-2.7 us; the shared memory is the tighter bound)
+constexpr long long COARSE_TOP = 120000;
+
+template <typename R>
+static CoarsePlan<R> coarse_plan(const wpf_handle* h, const Hierarchy<R>& H, int nu, long long big, int wfrom) {
+    CoarsePlan<R> p;
+    int lb = H.nlev - 1;   // first level of the plain V-cycle
+    while (lb > 0 && ncells(H.lv[lb - 1].g) <= vcycle_cells<R>()) --lb;
+    unsigned wmask = 0;
+    for (int l = 0; l < lb; ++l)
+        if (l >= wfrom && ncells(H.lv[l].g) < big) wmask |= 1u << l;
+    int nv = lb;
+    while (nv < H.nlev - 1 && ncells(H.lv[nv].g) > coarse_single<R>()) ++nv;
+    for (int l = 0; l < H.nlev; ++l) {
+        const Grid& g = H.lv[l].g;
+        const long long cells = ncells(g);
+        if (l < lb && (cells >= big || cells > COARSE_TOP)) continue;
+        p.l0 = l;
+        p.smem = coarse_fit(H, l, nv, wmask, nu, COARSE_MAXC, p.args);
+        if (p.smem) return p;
+    }
+    p.l0 = H.nlev;   // not reached: the last level (at most 2 cells per axis) always fits
+    return p;
+}
+
+template <typename R>
+static void launch_coarse(wpf_handle* h, CoarsePlan<R>& p, int cls, double* dot, cudaStream_t s) {
+    p.args.dot = dot;
+    p.args.err = reinterpret_cast<int*>(h->dsc + S_KERR);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p.args.C);
+    cfg.blockDim = dim3(coarse_nt<R>());
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)p.args.C;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    WPF_LAUNCH(h, cls, cudaLaunchKernelEx(&cfg, k_coarse<R>, p.args));
+}
+
+template <typename R>
+static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& plan, int nu, long long big,
                         int wfrom, double* rz, bool& need_dot) {
     cudaStream_t s = h->stream;
     const dim3 sb(SX, SY);
-    if (l >= lb) {
-        BottomArgs<R> A;
-        A.l0 = lb;
-        A.nlev = H.nlev;
-        A.nu = nu;
-        for (int q = 0; q < H.nlev; ++q) A.lv[q] = H.lv[q];
-        WPF_LAUNCH(h, lb == 0 ? KC_SMOOTH0 : KC_BOTTOM,
-                   k_bottom<R><<<1, BOTTOM_THREADS, bottom_smem(H, lb), s>>>(A));
+    if (l >= plan.l0) {
+        if (l == 0) need_dot = false;
+        launch_coarse(h, plan, l == 0 ? KC_SMOOTH0 : KC_BOTTOM, l == 0 ? rz : nullptr, s);
         return;
     }
     Level<R>& L = H.lv[l];
@@ -1616,7 +1487,7 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, int lb, int nu, l
         const R* pre_end = buf[(nu - 1) & 1];
         WPF_LAUNCH(h, KC_MGREST, k_resid_restrict<R><<<cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), 0, s>>>(
             g, C.g, L.cx, L.cy, L.cz, L.diag, pre_end, L.b, C.b));
-        cycle_level(h, H, l + 1, lb, nu, big, wfrom, nullptr, need_dot);
+        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr, need_dot);
         for (int it = 0; it < nu; ++it) {
             const int w = nu + it;   // sweep number in the cycle: writes buf[w & 1]
             R* in = buf[(w + 1) & 1];
@@ -1633,7 +1504,7 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, int lb, int nu, l
     for (int rep = 0; rep < gamma; ++rep) {
         WPF_LAUNCH(h, KC_MGREST, k_resid_restrict<R><<<cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), 0, s>>>(
             g, C.g, L.cx, L.cy, L.cz, L.diag, L.x, L.b, C.b));
-        cycle_level(h, H, l + 1, lb, nu, big, wfrom, nullptr, need_dot);
+        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr, need_dot);
         launch_prolong<R>(h, g, C.g, L.idiag, L.x, C.x, s);
         if (rep + 1 < gamma) {
             for (int it = 0; it < nu; ++it) half_post();
@@ -1647,12 +1518,9 @@ template <typename R>
 static void vcycle(wpf_handle* h, Hierarchy<R>& H, int nu, double* rz) {
     const long long big = h->opts.sweep_min_cells > 0 ? h->opts.sweep_min_cells : BIG_CELLS;
     const int wfrom = h->opts.w_from_level > 0 ? h->opts.w_from_level : 2;
-    int lb = H.nlev - 1;
-    while (lb > 0 && ncells(H.lv[lb - 1].g) <= bottom_cells<R>() &&
-           bottom_smem(H, lb - 1) <= BOTTOM_SMEM_MAX)
-        --lb;
+    CoarsePlan<R> plan = coarse_plan(h, H, nu, big, wfrom);
     bool need_dot = rz != nullptr;
-    cycle_level(h, H, 0, lb, nu, big, wfrom, rz, need_dot);
+    cycle_level(h, H, 0, plan, nu, big, wfrom, rz, need_dot);
     if (need_dot) {
         const Grid& g = H.lv[0].g;
         WPF_LAUNCH(h, KC_VEC, k_dot<R><<<row_blocks(h, g), RB, 0, h->stream>>>(g, H.r, H.z, rz));
@@ -1805,8 +1673,8 @@ static int pcg(wpf_handle* h, Hierarchy<R>& H, double tol, int maxit, int nu, in
 
 template <typename R>
 static int set_sweep_smem() {
-    WPF_CUDA(cudaFuncSetAttribute(k_bottom<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)BOTTOM_SMEM_MAX));
+    WPF_CUDA(cudaFuncSetAttribute(k_coarse<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COARSE_SMEM));
+    WPF_CUDA(cudaFuncSetAttribute(k_coarse<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     WPF_CUDA(cudaFuncSetAttribute(k_sweep_async<R, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sweep_smem<R>()));
     WPF_CUDA(cudaFuncSetAttribute(k_sweep_async<R, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
