@@ -110,8 +110,10 @@ struct CoarseArgs {
     int* err;                // set when a bounded wait ran out
 };
 
-// A cell's vectors: {a-, a+, b-, b+} and {c-, c+, 1/diag, rhs}, the couplings to
-// its six neighbours and the right-hand side times 1/diag.
+// A cell's vectors: {a-, a+, b-, b+} and {c-, c+, scale, rhs}, the couplings to
+// its six neighbours and the right-hand side times scale = 1/diag.  A dead cell
+// (1/diag = 0; flagged in the table) has scale 1: it is never relaxed, but where a
+// negative permeability left it couplings its residual counts.
 template <typename R>
 struct alignas(16) Quad {
     R v[4];
@@ -179,7 +181,7 @@ __device__ __forceinline__ int slab_begin(const CoarseLevel& L, int ncd, int C, 
 }
 __device__ __forceinline__ int slab_owner(int shift, int ncd, int C, int c) { return (((c >> shift) + 1) * C - 1) / ncd; }
 
-constexpr unsigned CT_ODD = 1u << 20, CT_LEFT = 1u << 21, CT_RIGHT = 1u << 22;
+constexpr unsigned CT_ODD = 1u << 20, CT_LEFT = 1u << 21, CT_RIGHT = 1u << 22, CT_DEAD = 1u << 23;
 
 // The part of a level that depends on the CTA.
 template <typename R>
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
     // halos [side][parity of the exchange]; rhs from the slabs at CTA 0; correction from CTA 0
     __shared__ uint64_t bars[6];
     __shared__ CoarseOp ops[COARSE_MAXOP];
+    __shared__ int coupled;   // a dead black cell has couplings (its residual is not zero)
     __shared__ unsigned char owner[COARSE_MAXK][2];   // CTAs of the children of a plane of level lx
     R* sm = reinterpret_cast<R*>(smem_raw);
     const int tid = threadIdx.x;
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
     if (tid == NT - 1) {
         for (int q = 0; q < 6; ++q) halo_bar_init(&bars[q]);
         halo_bar_fence();
+        coupled = 0;
     }
     __syncthreads();
     if (tid < nlev) coarse_level_init<R>(lv[tid], a.ncd, C, rank);
@@ -304,7 +308,15 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
             for (int u = 0; u < UN; ++u) {
                 if (lq[u] >= nlev) continue;
                 const CoarseLevel& L = lv[lq[u]];
-                const R id = ld[u][6];
+                const bool dead = ld[u][6] == (R)0;
+                const R id = dead ? (R)1 : ld[u][6];
+                if (dead) {
+                    place[u] |= CT_DEAD;
+                    bool c = ld[u][7] != (R)0;
+#pragma unroll
+                    for (int v = 0; v < 6; ++v) c = c || ld[u][v] != (R)0;
+                    if (c && at[u] >= L.NS) coupled = 1;
+                }
                 Quad<R> A, B;
 #pragma unroll
                 for (int v = 0; v < 4; ++v) A.v[v] = ld[u][v] * id;
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                 reinterpret_cast<Quad<R>*>(sm + L.oB)[at[u]] = B;
                 reinterpret_cast<unsigned*>(sm)[L.oT + at[u]] = place[u];
                 if (at[u] < L.NS) {
-                    sm[L.oD + at[u]] = ld[u][8];
+                    sm[L.oD + at[u]] = dead ? (R)1 : ld[u][8];
                     reinterpret_cast<unsigned*>(sm)[L.oP + at[u]] = parent[u];
                 }
             }
@@ -395,6 +407,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                     R* x;
                     const R *xa, *xbm, *xbp, *xcm, *xcp;
                     unsigned d, idx;
+                    bool dead;
                 } c0[K], c1[K];
                 auto fetch = [&](Cell& c, int cc, int m) {
                     const bool on = m < n;
@@ -407,6 +420,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                     c.idx = (unsigned)(cc * XS + o);
                     c.x = on ? X + c.idx : nullptr;
                     c.d = on ? d : 0u;
+                    c.dead = (d & CT_DEAD) != 0;
                     c.xa = O - ((d & CT_ODD) ? 0 : 1);
                     c.xbm = O - W;
                     c.xbp = O + W;
@@ -421,6 +435,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                         if (sizeof(R) == 8 && !c[q].x) continue;
                         val[q] = zero ? c[q].b.v[3]
                                       : quad_relax(c[q].a, c[q].b, c[q].xa, c[q].xbm, c[q].xbp, c[q].xcm, c[q].xcp);
+                        if (c[q].dead) val[q] = 0;
                     }
 #pragma unroll
                     for (int q = 0; q < K; ++q) {
@@ -455,6 +470,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                             const R* O = Y + o;
                             val = quad_relax(A[cc * NS + m], qb, O - ((d & CT_ODD) ? 0 : 1), O - W, O + W, O - PS, O + PS);
                         }
+                        if (d & CT_DEAD) val = 0;
                         X[cc * XS + o] = val;
                         mirror(d, (unsigned)(cc * XS) + o, val);
                     }
@@ -463,8 +479,8 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
             }
         } else if (op.kind == OP_RESTRICT || op.kind == OP_GATHER) {
             // right-hand side of the next level := residual summed over each aggregate
-            // (red cells: the black ones were relaxed last; the red cell of aggregate I
-            // in a row is the row's slot I).  To CTA 0, an aggregate whose second
+            // (red cells and coupled dead black ones: the other black ones were relaxed
+            // last; the cell of aggregate I in a row is the row's slot I).  To CTA 0, an aggregate whose second
             // plane is another CTA's gets that part in a second array.  With x* the
             // relaxed value of a cell, its residual is diag (x* - x).
             const CoarseLevel& Q = lv[op.l + 1];
@@ -484,8 +500,13 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
                     if (b >= nb || lp < 0 || lp >= cnt) continue;
                     const int t = (lp * nb + b) * hx + I;
                     const unsigned d = T[t], idx = d & (CT_ODD - 1);
-                    const R* O = X + XS + idx;
+                    const R* O = X + XS + idx;   // (below, the row's black slot: the red cells around it)
                     s += D[t] * (quad_relax(A[t], B[t], O - ((d & CT_ODD) ? 0 : 1), O - W, O + W, O - PS, O + PS) - X[idx]);
+                    if (!coupled) continue;
+                    const unsigned e = T[NS + t];
+                    if (!(e & CT_DEAD)) continue;
+                    O = X + (e & (CT_ODD - 1));
+                    s += quad_relax(A[NS + t], B[NS + t], O - ((e & CT_ODD) ? 0 : 1), O - W, O + W, O - PS, O + PS);
                 }
                 const int at = ((I + J + K + 1) & 1) * Q.NS + ((K - Q.c0) * Q.nb + J) * Q.hx + (I >> 1);
                 if (!gather) sm[Q.oB + at * 4 + 3] = s * sm[Q.oB + at * 4 + 2];
@@ -524,8 +545,8 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
             const unsigned* P = reinterpret_cast<const unsigned*>(sm) + L.oP;
             for (int m = tid; m < n; m += nt) {
                 const unsigned d = T[m], idx = d & (CT_ODD - 1);
-                const R add = sm[P[m]], id = B[m].v[2];
-                const R val = id == (R)0 ? (R)0 : X[idx] + add;
+                const R add = sm[P[m]];
+                const R val = d & CT_DEAD ? (R)0 : X[idx] + add;
                 X[idx] = val;
                 mirror(d, idx, val);
             }

@@ -1,0 +1,251 @@
+// wpf_diag.cuh -- the showProgress reductions (wPFAW3D.f90:1695, 1756-1810) of
+// wpf_reduce (pitched fields) and wpf_reduce_noalloc (dense arrays).
+//
+// What bounds it: two FP64 reads per cell, once the FP64 pipe (2 operations per
+// SM and clock) is left out.  Two compensated sums, five maxima and a distance
+// per cell were 25 FP64 operations, one block per plane and one thread over the
+// planes at the end: 553 + 189 us at 160^3.  Here a cell costs integer operations
+// only:
+//   * sum(1 - f) = N - S and sum(1 + f) = N + S with S = sum f taken exactly: f
+//     in units of 2^-61 as a 64-bit integer, its two halves added up apart (no
+//     rounding, so no order either; a term below 2^-9 loses what lies under
+//     2^-61, where 1 -+ f lost what lies under 2^-53).  |f| >= 2, Inf and NaN take
+//     a compensated FP64 sum instead;
+//   * maxima and minima compare ordered 64-bit keys (NaN ignored, as fmax does);
+//   * the distance to the reference cell is an integer number of cells squared.
+// Measured with the reduction of the block records by a warp per field: 160^3
+// 745 -> 38 us on the device, 771 -> 62 us a call.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+
+namespace wpf {
+namespace diag {
+
+constexpr int BLOCKS = 608;      // four on each of 152 SMs: one wave
+constexpr int THREADS = 256;
+enum Field { HI = 0, LO, SLOW_S, SLOW_C, DIST2, PMAX, PMIN, CMAX, CMIN, CORE, OMAX = CORE, FLUX_S, FLUX_C, FIELDS };
+
+typedef long long ll;
+typedef unsigned long long ull;
+
+// Order of doubles as order of signed integers (its own inverse).
+__host__ __device__ inline ll key_of_bits(ll b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+__host__ __device__ inline double value_of_key(ll k) {
+    const ll b = key_of_bits(k);
+    double v;
+#ifdef __CUDA_ARCH__
+    v = __longlong_as_double(b);
+#else
+    memcpy(&v, &b, 8);
+#endif
+    return v;
+}
+__host__ __device__ inline ll key_of(double v) {
+    ll b;
+#ifdef __CUDA_ARCH__
+    b = __double_as_longlong(v);
+#else
+    memcpy(&b, &v, 8);
+#endif
+    return key_of_bits(b);
+}
+
+__device__ __forceinline__ void two_sum(double& s, double& c, double v) {
+    const double t = s + v;
+    const double bp = t - s;
+    c += (s - (t - bp)) + (v - bp);
+    s = t;
+}
+
+// What a thread (then a warp, a block) has reduced.
+struct Acc {
+    ll hi = 0, dist2 = 0;
+    ull lo = 0;
+    double slow_s = 0.0, slow_c = 0.0;
+    ll pmax, pmin, cmax, cmin, omax;
+    double flux_s = 0.0, flux_c = 0.0;
+    __device__ __forceinline__ Acc() {
+        pmax = cmax = omax = key_of(-1.0e308);
+        pmin = cmin = key_of(1.0e308);
+    }
+    // a value against a running maximum and minimum (NaN ignored): the upper words
+    // decide nearly always, and a value equal to an extremum, as the untouched rock's,
+    // changes nothing
+    static __device__ __forceinline__ void extremum(double v, ll& mx, ll& mn) {
+        const int h = __double2hiint(v), s = h >> 31, kh = h ^ (s & 0x7fffffff);
+        const unsigned kl = (unsigned)(__double2loint(v) ^ s);
+        const int xh = (int)(mx >> 32), nh = (int)(mn >> 32);
+        if (kh > xh || kh < nh || (kh == xh && kl > (unsigned)mx) || (kh == nh && kl < (unsigned)mn)) {
+            if ((__double_as_longlong(v) & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) {
+                const ll k = (ll)kh << 32 | kl;
+                mx = k > mx ? k : mx;
+                mn = k < mn ? k : mn;
+            }
+        }
+    }
+    __device__ __forceinline__ void extrema(double f, double c) {
+        extremum(f, pmax, pmin);
+        extremum(c, cmax, cmin);
+    }
+    // an interior cell's phase, dist2 cells squared from the reference cell
+    __device__ __forceinline__ void interior(double f, ll d2) {
+        const unsigned h = (unsigned)__double2hiint(f), l = (unsigned)__double2loint(f);
+        const unsigned e = (h >> 20) & 0x7ffu, sh = 1023u - e;   // f = mantissa 2^-61 >> sh
+        if (sh < 32u) {   // 2^-31 <= |f| < 2
+            const unsigned mh = ((h & 0xfffffu) | 0x100000u) << 9 | l >> 23, ml = l << 9;
+            const unsigned vh = mh >> sh, vl = __funnelshift_r(ml, mh, sh);
+            const unsigned s = (unsigned)((int)h >> 31);
+            // two's complement of a negative value: lower word and carry apart
+            lo += (ull)(vl ^ s) + (s & 1u);
+            hi += (int)(vh ^ s);
+        } else if (e < 1024u) {
+            const ull m = ((((ull)h << 32 | l) & 0xfffffffffffffull) | 0x10000000000000ull) << 9;
+            const ll v = m >> (sh < 63u ? sh : 63u);
+            const ll w = (int)h < 0 ? -v : v;
+            lo += (unsigned)w;
+            hi += w >> 32;
+        } else {
+            two_sum(slow_s, slow_c, f);
+        }
+        if ((int)h >= 0 && (h | l) != 0 && d2 > dist2 && __double_as_longlong(f) <= 0x7ff0000000000000ll) dist2 = d2;   // f > 0
+    }
+    __device__ __forceinline__ void outlet(double f) {
+        const ll b = __double_as_longlong(f);
+        if ((b & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) {
+            const ll k = key_of_bits(b);
+            omax = k > omax ? k : omax;
+        }
+    }
+};
+
+// Two values of a field (or, for the compensated pairs, of its first word) as one.
+__device__ __forceinline__ ll fold(int field, ll a, ll b) {
+    switch (field) {
+        case PMAX: case CMAX: case OMAX: case DIST2: return a > b ? a : b;
+        case PMIN: case CMIN: return a < b ? a : b;
+        default: return a + b;
+    }
+}
+__device__ __forceinline__ bool is_pair(int field) { return field == SLOW_S || field == FLUX_S; }
+
+// One field over a warp; every lane gets it.  Compensated pairs fold word and
+// carry together (v2 the carry).
+__device__ __forceinline__ void warp_fold(int field, ll& v, ll& v2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const ll w = __shfl_xor_sync(0xffffffffu, v, o);
+        if (is_pair(field)) {
+            const ll w2 = __shfl_xor_sync(0xffffffffu, v2, o);
+            double s = __longlong_as_double(v), c = __longlong_as_double(v2);
+            two_sum(s, c, __longlong_as_double(w));
+            v = __double_as_longlong(s);
+            v2 = __double_as_longlong(c + __longlong_as_double(w2));
+        } else {
+            v = fold(field, v, w);
+        }
+    }
+}
+
+// The block's record: NF fields (CORE, or FIELDS with the handle's).
+template <int NF>
+__device__ __forceinline__ void store_record(const Acc& a, ll* __restrict__ rec) {
+    __shared__ ll sm[THREADS / 32][FIELDS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ll v[FIELDS] = {a.hi, (ll)a.lo, __double_as_longlong(a.slow_s), __double_as_longlong(a.slow_c), a.dist2,
+                    a.pmax, a.pmin, a.cmax, a.cmin, a.omax, __double_as_longlong(a.flux_s),
+                    __double_as_longlong(a.flux_c)};
+    // the FP64 folds (a chain of 64-cycle operations) run only where a thread has
+    // something to fold; below, an empty pair (all bits zero) is stepped over
+    const bool slow = __any_sync(0xffffffffu, (v[SLOW_S] | v[SLOW_C]) != 0);
+    const bool flux = __any_sync(0xffffffffu, (v[FLUX_S] | v[FLUX_C]) != 0);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        if (f == SLOW_C || f == FLUX_C) continue;
+        if ((f == SLOW_S && !slow) || (f == FLUX_S && !flux)) continue;
+        ll none = 0;
+        warp_fold(f, v[f], is_pair(f) ? v[f + 1] : none);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) sm[warp][f] = v[f];
+    __syncthreads();
+    if (threadIdx.x < NF && threadIdx.x != SLOW_C && threadIdx.x != FLUX_C) {
+        const int f = threadIdx.x;
+        ll s = sm[0][f], c = is_pair(f) ? sm[0][f + 1] : 0;
+        for (int w = 1; w < THREADS / 32; ++w) {
+            if (is_pair(f)) {
+                if ((sm[w][f] | sm[w][f + 1]) == 0) continue;
+                double ds = __longlong_as_double(s), dc = __longlong_as_double(c);
+                two_sum(ds, dc, __longlong_as_double(sm[w][f]));
+                s = __double_as_longlong(ds);
+                c = __double_as_longlong(dc + __longlong_as_double(sm[w][f + 1]));
+            } else {
+                s = fold(f, s, sm[w][f]);
+            }
+        }
+        rec[f] = s;
+        if (is_pair(f)) rec[f + 1] = c;
+    }
+}
+
+// n block records -> one: a warp per field.
+template <int NF>
+__device__ __forceinline__ void fold_records(const ll* __restrict__ rec, int n, ll* __restrict__ out) {
+    const int f = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (f >= NF || f == SLOW_C || f == FLUX_C) return;
+    constexpr int PER = (BLOCKS + 31) / 32;
+    // all of a lane's records in flight together; a lane without one repeats the
+    // first for an extremum and adds nothing to a sum
+    const bool sum = f == HI || f == LO || is_pair(f);
+    ll w[PER], w2[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int r = lane + 32 * q;
+        w[q] = r < n ? rec[(ll)r * NF + f] : (sum ? 0 : rec[f]);
+        w2[q] = is_pair(f) && r < n ? rec[(ll)r * NF + f + 1] : 0;
+    }
+    ll v = w[0], c = w2[0];
+#pragma unroll
+    for (int q = 1; q < PER; ++q) {
+        if (is_pair(f)) {
+            if ((w[q] | w2[q]) == 0) continue;
+            double ds = __longlong_as_double(v), dc = __longlong_as_double(c);
+            two_sum(ds, dc, __longlong_as_double(w[q]));
+            v = __double_as_longlong(ds);
+            c = __double_as_longlong(dc + __longlong_as_double(w2[q]));
+        } else {
+            v = fold(f, v, w[q]);
+        }
+    }
+    warp_fold(f, v, c);
+    if (lane == 0) {
+        out[f] = v;
+        if (is_pair(f)) out[f + 1] = c;
+    }
+}
+
+// The record's numbers on the host.
+struct Result {
+    double one_minus, one_plus, dist, pmax, pmin, cmax, cmin;   // sums, distance in cells
+};
+inline Result result(const ll* r, double cells) {
+    Result q;
+    const __int128 S = ((__int128)r[HI] << 32) + (__int128)(ull)r[LO], N = (__int128)cells << 61;
+    double slow, carry;
+    memcpy(&slow, &r[SLOW_S], 8);
+    memcpy(&carry, &r[SLOW_C], 8);
+    slow += carry;
+    q.one_minus = ldexp((double)(N - S), -61) - slow;
+    q.one_plus = ldexp((double)(N + S), -61) + slow;
+    q.dist = sqrt((double)r[DIST2]);
+    q.pmax = value_of_key(r[PMAX]);
+    q.pmin = value_of_key(r[PMIN]);
+    q.cmax = value_of_key(r[CMAX]);
+    q.cmin = value_of_key(r[CMIN]);
+    return q;
+}
+
+}  // namespace diag
+}  // namespace wpf

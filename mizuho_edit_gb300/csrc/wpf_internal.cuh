@@ -58,8 +58,8 @@ enum Slot {
     S_PQ,               // PCG p.q
     S_RR,               // PCG r.r
     S_RZ0, S_RZ1,       // PCG r.z (double buffered)
-    S_SUM0, S_SUM1, S_SUM2, S_SUM3,   // diagnostics
-    S_MAX0, S_MAX1, S_MAX2, S_MAX3, S_MAX4,
+    S_DIAG0,            // diagnostics: the record of wpf_diag.cuh and the reference pressure
+    S_DIAGN = S_DIAG0 + 12,
     S_NWORK,            // work-list counts of the fused update: interface cells and
                         // concentration-only cells (two ints in a double slot)
     S_WSS2,             // sum of the squared last increment (input scale of the learned start)
@@ -271,8 +271,7 @@ struct wpf_handle {
     bool snap_pending;
     double* dsc;             // device scalar slots
     double* hsc;             // pinned host mirror of the scalar slots
-    double* partials;        // per-block partial sums of the diagnostics
-    int npartials;
+    double* partials;        // block records of the diagnostics
     double taumin_last;      // taumin of the last phase-derivative pass
     int64_t bytes;           // device bytes allocated
     bool vel_valid;

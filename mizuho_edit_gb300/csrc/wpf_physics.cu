@@ -25,6 +25,7 @@
 // Divisions by a parameter (dx, mu, tau0) become multiplications by its
 // precomputed reciprocal; results differ from the literal Fortran arithmetic
 // by a few ulp, well inside the parity tolerances.
+#include "wpf_diag.cuh"
 #include "wpf_internal.cuh"
 
 namespace wpf {
@@ -861,84 +862,48 @@ int breakthrough_plane(const wpf_params& p) {
     return ix >= 1 ? ix : 1;
 }
 
-// showProgress reductions (:1695, :1756-1810): per-block partials of
-//   S0 = sum(1-phase), S1 = sum(1+phase)  (interior, compensated per thread)
-//   M0 = max r^2 over phase > 0, max/min phase, max/min concent (over G)
-//   S2 = inlet flux sum u_x(1->2) dx^2
-// then one block folds the partials in a fixed order.
+// showProgress reductions (wpf_diag.cuh) over the pitched fields, with the inlet
+// flux sum u_x(1->2) dx^2 and the maximum phase on the breakthrough plane: each
+// warp takes rows (j, k) of the halo grid, lanes along x.
 // ---------------------------------------------------------------------------
-struct DiagPart {
-    double s0, c0, s1, c1, s2, c2, r2max, pmax, pmin, cmax, cmin, omax;
-};
-
-__device__ __forceinline__ void two_sum(double& s, double& c, double v) {
-    const double t = s + v;
-    const double bp = t - s;
-    c += (s - (t - bp)) + (v - bp);
-    s = t;
-}
-
-__global__ void k_diag_partial(Grid g, Phys P, int ix_ref, int iy_ref, int iz_ref, int ix_bt,
-                               const double* __restrict__ ph, const double* __restrict__ cc,
-                               const double* __restrict__ pr, const double* __restrict__ Tx,
-                               DiagPart* __restrict__ out) {
-    // one block per plane k (0..nz+1), threads over rows j and x
-    __shared__ double sm[32];
-    const int k = blockIdx.x;
-    double s0 = 0, c0 = 0, s1 = 0, c1 = 0, s2 = 0, c2 = 0, r2max = 0;
-    double pmax = -1.0e308, pmin = 1.0e308, cmax = -1.0e308, cmin = 1.0e308, omax = -1.0e308;
-    const double dx = P.dx;
-    const double xref = dx * (ix_ref - 1) + 0.5 * dx, yref = dx * (iy_ref - 1) + 0.5 * dx,
-                 zref = dx * (iz_ref - 1) + 0.5 * dx;
-    for (int j = threadIdx.y; j <= g.ny + 1; j += blockDim.y)
-        for (int i = threadIdx.x; i <= g.nx + 1; i += blockDim.x) {
-            const long long n = g.at(i, j, k);
-            const double f = ph[n], c = cc[n];
-            pmax = fmax(pmax, f); pmin = fmin(pmin, f);
-            cmax = fmax(cmax, c); cmin = fmin(cmin, c);
-            const bool interior = i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
-            if (interior) {
-                two_sum(s0, c0, 1.0 - f);
-                two_sum(s1, c1, 1.0 + f);
-                if (f > 0.0) {
-                    const double x = dx * (i - 1) + 0.5 * dx - xref, y = dx * (j - 1) + 0.5 * dx - yref,
-                                 z = dx * (k - 1) + 0.5 * dx - zref;
-                    r2max = fmax(r2max, x * x + y * y + z * z);
-                }
-                if (i == 1 && g.nx >= 2) {
-                    const double u = -(Tx[n] * ((pr[n + 1] - pr[n]) * P.inv_dx));
-                    two_sum(s2, c2, u * dx * dx);
-                }
-                if (i == ix_bt) omax = fmax(omax, f);   // breakthrough plane
+__global__ void __launch_bounds__(diag::THREADS) k_diag(Grid g, Phys P, int ix_ref, int iy_ref, int iz_ref, int ix_bt,
+                                                        const double* __restrict__ ph, const double* __restrict__ cc,
+                                                        const double* __restrict__ pr, const double* __restrict__ Tx,
+                                                        long long* __restrict__ rec) {
+    diag::Acc a;
+    const int lane = threadIdx.x & 31;
+    const int rows = (g.ny + 2) * (g.nz + 2), step = gridDim.x * (diag::THREADS / 32);
+    for (int r = blockIdx.x * (diag::THREADS / 32) + (threadIdx.x >> 5); r < rows; r += step) {
+        const int k = r / (g.ny + 2), j = r - k * (g.ny + 2);
+        const bool in = j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
+        const long long dj = j - iy_ref, dk = k - iz_ref, jk2 = dj * dj + dk * dk;
+        const long long n0 = g.at(0, j, k);
+#pragma unroll 4
+        for (int i = lane; i <= g.nx + 1; i += 32) {
+            const double f = ph[n0 + i], c = cc[n0 + i];
+            a.extrema(f, c);
+            if (in && i >= 1 && i <= g.nx) {
+                const long long di = i - ix_ref;
+                a.interior(f, jk2 + di * di);
+                if (i == ix_bt) a.outlet(f);
             }
         }
-    DiagPart r;
-    r.s0 = block_sum(s0, sm); r.c0 = block_sum(c0, sm);
-    r.s1 = block_sum(s1, sm); r.c1 = block_sum(c1, sm);
-    r.s2 = block_sum(s2, sm); r.c2 = block_sum(c2, sm);
-    r.r2max = block_max(r2max, sm, 0.0);
-    r.pmax = block_max(pmax, sm, -1.0e308); r.pmin = block_min(pmin, sm, 1.0e308);
-    r.cmax = block_max(cmax, sm, -1.0e308); r.cmin = block_min(cmin, sm, 1.0e308);
-    r.omax = block_max(omax, sm, -1.0e308);
-    if (threadIdx.x == 0 && threadIdx.y == 0) out[k] = r;
+    }
+    // the inlet plane with full warps along y: one lane per row in the loop above
+    // would hold the FP64 pipe as long as 32 do
+    if (g.nx >= 2)
+        for (int t = blockIdx.x * diag::THREADS + threadIdx.x; t < g.ny * g.nz; t += gridDim.x * diag::THREADS) {
+            const long long n = g.at(1, 1 + t % g.ny, 1 + t / g.ny);
+            diag::two_sum(a.flux_s, a.flux_c, -(Tx[n] * ((pr[n + 1] - pr[n]) * P.inv_dx)) * P.dx * P.dx);
+        }
+    diag::store_record<diag::FIELDS>(a, rec + (long long)blockIdx.x * diag::FIELDS);
 }
 
-__global__ void k_diag_final(const DiagPart* __restrict__ parts, int nparts, double* out) {
-    if (threadIdx.x != 0) return;
-    double s0 = 0, c0 = 0, s1 = 0, c1 = 0, s2 = 0, c2 = 0, r2 = 0;
-    double pmax = -1.0e308, pmin = 1.0e308, cmax = -1.0e308, cmin = 1.0e308, omax = -1.0e308;
-    for (int q = 0; q < nparts; ++q) {
-        const DiagPart& p = parts[q];
-        two_sum(s0, c0, p.s0); c0 += p.c0;
-        two_sum(s1, c1, p.s1); c1 += p.c1;
-        two_sum(s2, c2, p.s2); c2 += p.c2;
-        r2 = fmax(r2, p.r2max);
-        pmax = fmax(pmax, p.pmax); pmin = fmin(pmin, p.pmin);
-        cmax = fmax(cmax, p.cmax); cmin = fmin(cmin, p.cmin);
-        omax = fmax(omax, p.omax);
-    }
-    out[0] = s0 + c0; out[1] = s1 + c1; out[2] = s2 + c2; out[3] = r2;
-    out[4] = pmax; out[5] = pmin; out[6] = cmax; out[7] = cmin; out[8] = omax;
+// The block records as one, and the reference cell's pressure (0 without one) behind it.
+__global__ void k_diag_final(const long long* __restrict__ rec, int n, const double* __restrict__ pref,
+                             long long* __restrict__ out) {
+    diag::fold_records<diag::FIELDS>(rec, n, out);
+    if (threadIdx.x == 0) out[diag::FIELDS] = pref ? __double_as_longlong(*pref) : 0ll;
 }
 
 // ---------------------------------------------------------------------------
@@ -1200,40 +1165,41 @@ int phys_set_dirichlet(wpf_handle* h) {
 
 int phys_reduce(wpf_handle* h, wpf_diag* d) {
     const Grid& g = h->g;
-    const int nparts = g.nz + 2;
-    if (h->npartials < nparts) {
-        if (h->partials) cudaFree(h->partials);
-        h->partials = nullptr;
-        int rc = dev_alloc(h, (void**)&h->partials, sizeof(DiagPart) * nparts + 64);
+    if (!h->partials) {
+        int rc = dev_alloc(h, (void**)&h->partials, sizeof(long long) * diag::BLOCKS * diag::FIELDS);
         if (rc) return rc;
-        h->npartials = nparts;
     }
-    DiagPart* parts = reinterpret_cast<DiagPart*>(h->partials);
-    WPF_LAUNCH(h, KC_OTHER, k_diag_partial<<<nparts, dim3(32, 8), 0, h->stream>>>(
-        g, h->phys, h->prm.ix_ref, h->prm.iy_ref, h->prm.iz_ref, breakthrough_plane(h->prm), h->phase,
-        h->concent, h->pressure, h->T[0], parts));
-    WPF_LAUNCH(h, KC_OTHER, k_diag_final<<<1, 32, 0, h->stream>>>(parts, nparts, h->dsc + S_SUM0));
-    WPF_CUDA(cudaGetLastError());
-    WPF_CUDA(cudaMemcpyAsync(h->hsc + S_SUM0, h->dsc + S_SUM0, 9 * sizeof(double),
-                             cudaMemcpyDeviceToHost, h->stream));
-    double pref = 0.0;
+    long long* rec = reinterpret_cast<long long*>(h->partials);
+    const long long rows = (long long)(g.ny + 2) * (g.nz + 2), want = (rows + diag::THREADS / 32 - 1) / (diag::THREADS / 32);
+    const int blocks = (int)(want < diag::BLOCKS ? want : diag::BLOCKS);
     const wpf_params& p = h->prm;
-    if (p.ix_ref >= 1 && p.ix_ref <= g.nx && p.iy_ref >= 1 && p.iy_ref <= g.ny && p.iz_ref >= 1 &&
-        p.iz_ref <= g.nz) {
-        WPF_CUDA(cudaMemcpyAsync(&pref, h->pressure + g.at(p.ix_ref, p.iy_ref, p.iz_ref),
-                                 sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    }
+    const bool ref = p.ix_ref >= 1 && p.ix_ref <= g.nx && p.iy_ref >= 1 && p.iy_ref <= g.ny && p.iz_ref >= 1 &&
+                     p.iz_ref <= g.nz;
+    WPF_LAUNCH(h, KC_OTHER, k_diag<<<blocks, diag::THREADS, 0, h->stream>>>(
+        g, h->phys, p.ix_ref, p.iy_ref, p.iz_ref, breakthrough_plane(p), h->phase, h->concent, h->pressure, h->T[0],
+        rec));
+    WPF_LAUNCH(h, KC_OTHER, k_diag_final<<<1, 32 * diag::FIELDS, 0, h->stream>>>(
+        rec, blocks, ref ? h->pressure + g.at(p.ix_ref, p.iy_ref, p.iz_ref) : nullptr,
+        reinterpret_cast<long long*>(h->dsc + S_DIAG0)));
+    WPF_CUDA(cudaGetLastError());
+    WPF_CUDA(cudaMemcpyAsync(h->hsc + S_DIAG0, h->dsc + S_DIAG0, (diag::FIELDS + 1) * sizeof(double),
+                             cudaMemcpyDeviceToHost, h->stream));
     WPF_CUDA(cudaStreamSynchronize(h->stream));
-    const double* o = h->hsc + S_SUM0;
+    long long r[diag::FIELDS + 1];
+    memcpy(r, h->hsc + S_DIAG0, sizeof(r));
+    const diag::Result q = diag::result(r, (double)g.nx * g.ny * g.nz);
     const double dx = h->phys.dx;
-    d->pv = dx * dx * dx * p.porosity * 0.5 * o[0];
-    d->vcal = dx * dx * dx * (1.0 - p.porosity) * 0.5 * o[1];
-    d->inlet_flux = o[2];
-    d->rwhmax = sqrt(o[3]);
-    d->phase_max = o[4]; d->phase_min = o[5];
-    d->concent_max = o[6]; d->concent_min = o[7];
-    d->phase_max_outlet = o[8];
-    d->pressure_ref = pref;
+    double flux, carry;
+    memcpy(&flux, &r[diag::FLUX_S], 8);
+    memcpy(&carry, &r[diag::FLUX_C], 8);
+    d->pv = dx * dx * dx * p.porosity * 0.5 * q.one_minus;
+    d->vcal = dx * dx * dx * (1.0 - p.porosity) * 0.5 * q.one_plus;
+    d->inlet_flux = flux + carry;
+    d->rwhmax = fabs(dx) * q.dist;
+    d->phase_max = q.pmax; d->phase_min = q.pmin;
+    d->concent_max = q.cmax; d->concent_min = q.cmin;
+    d->phase_max_outlet = diag::value_of_key(r[diag::OMAX]);
+    memcpy(&d->pressure_ref, &r[diag::FIELDS], 8);
     return WPF_OK;
 }
 
