@@ -6,19 +6,15 @@
 // x, y, z); weights bf16 [Cout][27][Cin], tap t = (dz+1)*9 + (dy+1)*3 + (dx+1);
 // FP32 master weights, gradients and Adam moments.
 //
-// Convolution = implicit GEMM on tcgen05: one CTA of 128 threads owns 128
-// output voxels (M = 128, one TMEM lane each) and all Cout channels (N =
-// Cout); the K loop runs over the 27 taps, each tap one stage of K = Cin
-// (Cin/16 MMAs of K = 16).  Threads gather the A rows (the Cin channels of the
-// shifted voxel: Cin/8 16-byte chunks) and the B rows (weights of the tap)
-// into shared memory in the no-swizzle K-major core-matrix layout (8 rows x
-// 16 bytes per core matrix; LBO = byte stride between core matrices along K,
-// SBO = along M/N), two stages in flight: thread 0 issues the MMAs of a stage
-// and commits them to the stage's mbarrier, which the gatherers wait on
-// before refilling that buffer.  The FP32 accumulator lives in TMEM and is
-// read back with tcgen05.ld for the epilogue (bias, ReLU, bf16 store).
-// Weight gradient = the same machinery with M = (tap, Cin) rows, N = Cout and
-// K = voxels (split over CTAs, FP32 atomics into the gradient).  Data
+// Convolution = implicit GEMM on tcgen05 (k_conv3d_tile): one CTA owns a brick of
+// 8 x 16 output voxels (M = 128, one TMEM lane each) and all Cout channels (N =
+// Cout); the 27 taps are 27 x Cin/16 MMAs of K = 16 into one accumulator.  The
+// brick's input halo is staged once, each 8-channel chunk in planes of its own,
+// so that 8 consecutive x voxels form one core matrix (8 rows x 16 bytes) of the
+// no-swizzle K-major layout and every tap's A operand is a window of them; the
+// FP32 accumulator lives in TMEM and is read back with tcgen05.ld for the
+// epilogue (bias, ReLU, bf16 store).  Weight gradient (k_conv3d_wgrad) = the same
+// staged planes read the other way, K = voxels (MN-major operands).  Data
 // gradient = the forward kernel with the flipped, transposed weights.
 #include <cuda_bf16.h>
 #include <math.h>
@@ -122,16 +118,112 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// Shared memory of a conv CTA: two stages of A (128 rows) and B (COUT rows),
-// plus 1 KB so that every descriptor-addressed read stays inside the
-// allocation.  Sized per shape: the 16-channel layers take 10 KB, so many
-// CTAs share an SM and hide each other's gather latency.
-constexpr int CONV_SMEM_MAX = 96 * 1024;
+// ---- bricks ---------------------------------------------------------------------
+// A brick is 8 (x) by 16 (q: y, or z, whichever pads the grid less) voxels of one
+// plane of the third axis p.  Its halo is 10 x 18 x 3 voxels.  With 8 voxels per
+// row of the brick a group of 8 MMA rows is one row of it, the groups lie one
+// halo row apart, and no tap needs a copy of its own (bricks of 16 and more
+// voxels in x needed three copies shifted in x: 74 KB against 17 KB for 16
+// channels).  The threads stage it with 16-byte cp.async, the chunks of a voxel on
+// neighbouring lanes (bulk-tensor boxes of 8 channels measured the same, and
+// their 128-byte planes put a voxel's chunks on the same banks).
+constexpr int BK_X = 8, BK_Q = 16;
+constexpr int BOX_X = BK_X + 2, BOX_Q = BK_Q + 2;
+constexpr int ROWB = BOX_X * 16;                         // bytes of a halo row of one chunk
+// a plane of one chunk; 16 bytes more than the rows keep the chunks of a voxel on
+// different banks.  Plane p of chunk c is the (p CH + c)-th.
+constexpr int PLB = BOX_Q * ROWB + 16;
+constexpr int GPB = BK_X * BK_Q * 16 + 16;               // a chunk's plane of a brick without halo
+
+struct Brick {
+    int nx, ny, nz;
+    int ntx, nty, ntz, along_z;      // stacks per axis; q is z
+    int nb;                          // bricks of a stack (planes of p)
+    __device__ __forceinline__ void origin(int t, int& x, int& y, int& z) const {
+        const int r = t / ntx;
+        x = (t - r * ntx) * BK_X;
+        z = r / nty;
+        y = r - z * nty;
+        z *= along_z ? BK_Q : nb;
+        y *= along_z ? nb : BK_Q;
+    }
+    int count() const { return ntx * nty * ntz; }
+};
+
+// most: bricks that a stack may have; it gets as many as leave `want` stacks
+static Brick make_brick(int nx, int ny, int nz, int most, int want) {
+    auto up = [](long long a, int b) { return (a + b - 1) / b; };
+    Brick b;
+    b.nx = nx; b.ny = ny; b.nz = nz;
+    b.along_z = up(nz, BK_Q) * ny < up(ny, BK_Q) * nz;
+    b.ntx = (int)up(nx, BK_X);
+    const long long one = b.ntx * (b.along_z ? (long long)up(nz, BK_Q) * ny : (long long)up(ny, BK_Q) * nz);
+    b.nb = one / want < 1 ? 1 : (one / want > most ? most : (int)(one / want));
+    b.nty = b.along_z ? (int)up(ny, b.nb) : (int)up(ny, BK_Q);
+    b.ntz = b.along_z ? (int)up(nz, BK_Q) : (int)up(nz, b.nb);
+    return b;
+}
+
+static int sm_count() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        n = v > 0 ? v : 1;
+    }
+    return n;
+}
+
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool ok) {   // zeros when !ok
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// np planes of voxels with H layers of halo in x and q, from plane p0 - H on (zeros
+// outside the grid), by CT threads.  A thread keeps its place in the plane.
+template <int C, int H>
+__device__ __forceinline__ void stage(unsigned char* dst, const bf16_t* __restrict__ src, const Brick& b, int x0, int y0,
+                                      int z0, int np, int tid) {
+    constexpr int CH = C / 8, NX = BK_X + 2 * H, NQ = BK_Q + 2 * H;
+    constexpr int PL = H ? PLB : GPB;
+    const int p0 = (b.along_z ? y0 : z0) - H, pn = b.along_z ? b.ny : b.nz;
+    const long long ps = (b.along_z ? (long long)b.nx : (long long)b.nx * b.ny) * C;
+    const long long qs = (b.along_z ? (long long)b.nx * b.ny : (long long)b.nx) * C;
+    const int q0 = (b.along_z ? z0 : y0) - H, qn = b.along_z ? b.nz : b.ny;
+#pragma unroll 1   // (straight-line code runs at the speed of instruction fetch here)
+    for (int u = tid; u < NQ * NX * CH; u += CT) {
+        const int c = u % CH, v = u / CH, bx = v % NX, q = v / NX, x = x0 - H + bx;
+        const bool in = (unsigned)x < (unsigned)b.nx && (unsigned)(q0 + q) < (unsigned)qn;
+        const bf16_t* s = src + (q0 + q) * qs + (long long)x * C + 8 * c + p0 * ps;
+        unsigned char* d = dst + c * PL + (q * NX + bx) * 16;
+#pragma unroll 1
+        for (int p = 0; p < np; ++p, s += ps, d += CH * PL) {
+            const bool ok = in && (unsigned)(p0 + p) < (unsigned)pn;
+            copy16(d, ok ? s : src, ok);
+        }
+    }
+}
+
+// Weights: small ones (up to 28 KB: 16 <-> 16, 32) sit whole in shared memory; of
+// the others each tap is a stage of a ring.
 template <int CIN, int COUT>
-constexpr int conv_smem() { return 2 * (CIN * 256 + COUT * CIN * 2) + 1024; }
-constexpr int WG_STAGE_ = 32;
-template <int CIN, int COUT>
-constexpr int wgrad_smem() { return 2 * (128 * WG_STAGE_ * 2 + COUT * WG_STAGE_ * 2) + 1024; }
+struct ConvTile {
+    static constexpr int CH = CIN / 8;
+    static constexpr int WPL = COUT * 16 + 16;            // a chunk of a tap (bank padding as above)
+    static constexpr int TAP = CH * WPL;
+    static constexpr bool RES = 27 * CIN * COUT * 2 <= 28 * 1024;
+    static constexpr int NST = RES ? 1 : 4;
+    static constexpr int MOST = RES ? 4 : 2;              // bricks of a stack
+    static constexpr int abytes(int nb) { return (nb + 2) * CH * PLB; }
+    static constexpr int smem(int nb) { return abytes(nb) + (RES ? 27 : NST) * TAP + 1024; }
+    static_assert(smem(MOST) <= 200 * 1024, "conv stack exceeds shared memory");
+};
 
 struct ConvArgs {
     int nx, ny, nz, nvox;
@@ -144,104 +236,167 @@ struct ConvArgs {
     int* err;
 };
 
+// A CTA owns a stack of b.nb bricks, neighbours along p, with an accumulator
+// each: they share the halo planes between them and every tap's weights, which
+// all CTAs read from the same few L2 lines at the same time.  Four warps stage
+// and, at the end, read the accumulators; a fifth issues the MMAs.  Measured
+// against a CTA that gathered every tap and, for 16 channels, bricks of 16 and
+// more voxels in x: 64 -> 64 channels, 36x28x21 68 -> 32 us; 64^3, 16 -> 16
+// channels 40 -> 23 us; 16^3, 64 -> 64 46 -> 15 us.  What bounds it now: with 16
+// channels the MMAs themselves (~130 cycles each in the no-swizzle layout,
+// whatever the planes' alignment), with 64 the ring of taps (0.35 us each).
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT) k_conv3d(ConvArgs a) {
+__global__ void __launch_bounds__(CT + 32) k_conv3d_tile(ConvArgs a, Brick b) {
+    using T = ConvTile<CIN, COUT>;
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar_d, bar_w[T::NST], bar_e[T::NST];   // MMAs done; a tap (and all before it) landed / used
     __shared__ uint32_t tmem_sh;
-    constexpr int AB = CIN * 256;        // 128 rows x CIN bf16
-    constexpr int BB = COUT * CIN * 2;   // COUT rows x CIN bf16
-    constexpr int SB = AB + BB;
-    static_assert(2 * SB + 1024 == conv_smem<CIN, COUT>() && conv_smem<CIN, COUT>() <= CONV_SMEM_MAX,
-                  "conv stages exceed the shared allocation");
-    constexpr uint32_t NCOL = COUT < 32 ? 32 : COUT;
+    constexpr uint32_t NCOL = T::MOST * COUT;   // 64 or 128
     constexpr uint32_t IDESC = idesc_bf16(128, COUT);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, nb = b.nb;
     if (warp == 0) tmem_alloc(&tmem_sh, NCOL);
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+    if (tid == CT) {
+        mbar_init(&bar_d, 1);
+        for (int q = 0; q < T::NST; ++q) {
+            mbar_init(&bar_w[q], CT);
+            mbar_init(&bar_e[q], 1);
+        }
         fence_mbar_init();
     }
+    int x0, y0, z0;
+    b.origin(blockIdx.x, x0, y0, z0);
+    unsigned char* Bs = sm + T::abytes(nb);
     tc_before();
     __syncthreads();
     tc_after();
     const uint32_t tmem = tmem_sh;
     const uint32_t sbase = smem_u32(sm);
-
-    const long long v = (long long)blockIdx.x * CT + tid;   // output voxel of row m = tid
-    const bool vok = v < a.nvox;
-    int x = 0, y = 0, z = 0;
-    if (vok) {
-        x = (int)(v % a.nx);
-        const long long r = v / a.nx;
-        y = (int)(r % a.ny);
-        z = (int)(r / a.ny);
-    }
     bool ok = true;
-    for (int t = 0; t < 27; ++t) {
-        const int buf = t & 1;
-        if (t >= 2 && !mbar_wait(&bar[buf], ((t - 2) >> 1) & 1)) ok = false;
-        unsigned char* A = sm + buf * SB;
-        unsigned char* B = A + AB;
-        const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-        const int xs = x + dx, ys = y + dy, zs = z + dz;
-        const bool inb = vok && xs >= 0 && xs < a.nx && ys >= 0 && ys < a.ny && zs >= 0 && zs < a.nz;
-        const uint4* src =
-            reinterpret_cast<const uint4*>(a.in + (((long long)zs * a.ny + ys) * a.nx + xs) * CIN);
+    if (tid < CT) {
+        stage<CIN, 1>(sm, a.in, b, x0, y0, z0, nb + 2, tid);
+        auto landed = [&](int t) {   // this thread's part of tap t and of what came before it
+            fence_async_smem();
+            mbar_arrive(&bar_w[t % T::NST]);
+        };
+        // 16-byte pieces of a tap, piece u = (co, chunk): a thread keeps its pieces (or
+        // its piece of every TT-th tap) and walks the taps by constant steps; with a
+        // warp per scheduler index arithmetic here was most of the kernel's time
+        constexpr int PER = COUT * T::CH, NP = PER / CT > 0 ? PER / CT : 1, TT = CT / PER > 0 ? CT / PER : 1;
+        static_assert(PER % CT == 0 || CT % PER == 0, "pieces of a tap over the threads");
+        const bf16_t* src[NP];
+        unsigned char* dst[NP];
 #pragma unroll
-        for (int c = 0; c < CIN / 8; ++c) {
-            const uint4 q = inb ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(A + c * 2048 + (tid >> 3) * 128 + (tid & 7) * 16) = q;
+        for (int p = 0; p < NP; ++p) {
+            const int u = (tid + p * CT) % PER, c = u % T::CH, co = u / T::CH;
+            src[p] = a.w + ((long long)co * 27 + tid / PER) * CIN + 8 * c;
+            dst[p] = Bs + (T::RES ? tid / PER * T::TAP : 0) + c * T::WPL + co * 16;
         }
-        for (int q = tid; q < COUT * CIN / 8; q += CT) {
-            const int co = q / (CIN / 8), c = q - co * (CIN / 8);
-            const uint4 val = reinterpret_cast<const uint4*>(a.w + ((long long)co * 27 + t) * CIN)[c];
-            *reinterpret_cast<uint4*>(B + c * (COUT * 16) + (co >> 3) * 128 + (co & 7) * 16) = val;
+        if (T::RES) {
+#pragma unroll 1
+            for (int t = tid / PER; t < 27; t += TT)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    copy16(dst[p], src[p], true);
+                    dst[p] += TT * T::TAP;
+                    src[p] += TT * CIN;
+                }
+            copy_commit();
+            copy_wait<0>();
+            landed(0);
+        } else {
+#pragma unroll 1
+            for (int t = 0; t < 27; ++t) {
+                const int s = t % T::NST;
+                if (t >= T::NST && ok && !mbar_wait(&bar_e[s], (t / T::NST - 1) & 1)) ok = false;
+                if (ok)
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        copy16(dst[p] + s * T::TAP, src[p], true);
+                        src[p] += CIN;
+                    }
+                copy_commit();
+                if (t >= 2) {
+                    copy_wait<2>();
+                    landed(t - 2);
+                }
+            }
+            copy_wait<0>();
+            landed(25);
+            landed(26);
         }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
+    } else if (tid == CT) {
+        // descriptors advance by their 16-byte units (the address field has room for all of shared memory)
+        const uint64_t a0 = sdesc(sbase, PLB, ROWB), b0 = sdesc(sbase + T::abytes(nb), T::WPL, 128);
+        const uint32_t s9 = (b.along_z ? ROWB : T::CH * PLB) / 16, s3 = (b.along_z ? T::CH * PLB : ROWB) / 16;
+        uint32_t at = 0, row = 0;
+        int dx = 0, dy = 0;
+#pragma unroll 1
+        for (int t = 0; t < 27 && ok; ++t) {
+            const int s = T::RES ? 0 : t % T::NST;
+            if ((!T::RES || t == 0) && !mbar_wait(&bar_w[s], (t / T::NST) & 1)) {
+                ok = false;
+                break;
+            }
             tc_after();
+            const uint64_t bt = b0 + (uint32_t)(T::RES ? t : s) * (T::TAP / 16);
+            uint64_t ak = a0 + at;
+            uint32_t d = tmem;
+#pragma unroll 1
+            for (int k = 0; k < nb; ++k, d += COUT, ak += T::CH * PLB / 16)
 #pragma unroll
-            for (int kk = 0; kk < CIN / 16; ++kk) {
-                const uint64_t ad = sdesc(sbase + buf * SB + 2 * kk * 2048, 2048, 128);
-                const uint64_t bd = sdesc(sbase + buf * SB + AB + 2 * kk * (COUT * 16), COUT * 16, 128);
-                mma_bf16(tmem, ad, bd, IDESC, (t > 0 || kk > 0) ? 1u : 0u);
+                for (int kk = 0; kk < CIN / 16; ++kk)
+                    mma_bf16(d, ak + 2 * kk * (PLB / 16), bt + 2 * kk * (T::WPL / 16), IDESC, (t > 0 || kk > 0) ? 1u : 0u);
+            if (!T::RES) mma_commit(&bar_e[s]);
+            ++at;
+            if (++dx == 3) {
+                dx = 0;
+                at = row += s3;
+                if (++dy == 3) {
+                    dy = 0;
+                    at = row += s9 - 3 * s3;
+                }
             }
-            mma_commit(&bar[buf]);
         }
+        mma_commit(&bar_d);   // arrives when every MMA issued above has finished (or at once)
     }
-    // the last commit (tap 26: buffer 0, its 14th phase) covers every MMA
-    if (!mbar_wait(&bar[0], 1)) ok = false;
+    __syncwarp();
+    if (!mbar_wait(&bar_d, 0)) ok = false;
+    ok = __syncthreads_and(ok);
     tc_after();
+    if (tid < CT) {
+        const int q = tid / BK_X, x = x0 + tid % BK_X;
+        for (int k = 0; k < nb; ++k) {
+            const int y = y0 + (b.along_z ? k : q), z = z0 + (b.along_z ? q : k);
+            const bool in = x < b.nx && y < b.ny && z < b.nz;
+            const long long v = ((long long)z * b.ny + y) * b.nx + x;
+#pragma unroll 1
+            for (int c0 = 0; c0 < COUT; c0 += 16) {
+                float acc[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(k * COUT + c0), acc);
+                if (!ok || !in) continue;
 #pragma unroll
-    for (int c0 = 0; c0 < COUT; c0 += 16) {
-        float acc[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-        if (vok && ok) {
+                for (int i = 0; i < 16; ++i) {
+                    float s = acc[i] + (a.bias ? a.bias[c0 + i] : 0.f);
+                    if (a.relu) s = fmaxf(s, 0.f);
+                    acc[i] = s;
+                }
+                if (a.out16) {
+                    uint4* dst = reinterpret_cast<uint4*>(a.out16 + v * COUT + c0);
+                    dst[0] = make_uint4(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]), pack2(acc[4], acc[5]),
+                                        pack2(acc[6], acc[7]));
+                    dst[1] = make_uint4(pack2(acc[8], acc[9]), pack2(acc[10], acc[11]), pack2(acc[12], acc[13]),
+                                        pack2(acc[14], acc[15]));
+                } else {
+                    float4* dst = reinterpret_cast<float4*>(a.out32 + v * COUT + c0);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float s = acc[i] + (a.bias ? a.bias[c0 + i] : 0.f);
-                if (a.relu) s = fmaxf(s, 0.f);
-                acc[i] = s;
-            }
-            if (a.out16) {
-                uint4* dst = reinterpret_cast<uint4*>(a.out16 + v * COUT + c0);
-                dst[0] = make_uint4(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]), pack2(acc[4], acc[5]),
-                                    pack2(acc[6], acc[7]));
-                dst[1] = make_uint4(pack2(acc[8], acc[9]), pack2(acc[10], acc[11]), pack2(acc[12], acc[13]),
-                                    pack2(acc[14], acc[15]));
-            } else {
-                float4* dst = reinterpret_cast<float4*>(a.out32 + v * COUT + c0);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    dst[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+                    for (int i = 0; i < 4; ++i)
+                        dst[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+                }
             }
         }
     }
-    if (!ok) {   // a wait ran out: give the MMAs in flight a second bounded wait
-        mbar_wait(&bar[0], 1);
+    if (!ok) {   // a wait ran out: the MMAs in flight get a second bounded wait
+        mbar_wait(&bar_d, 0);
         if (tid == 0) atomicExch(a.err, 1);
     }
     tc_before();
@@ -249,297 +404,162 @@ __global__ void __launch_bounds__(CT) k_conv3d(ConvArgs a) {
     if (warp == 0) tmem_dealloc(tmem, NCOL);
 }
 
-// ---- row-tiled convolution of 16-channel inputs, staged by TMA ----------------
-// For a level whose nx is a multiple of TX (128, 64, 32 or 16) and whose ny
-// is a multiple of TY = 128 / TX, a CTA owns the TX x TY x 1 brick of output
-// voxels (x0.., y0.., z0): M = 128 rows in x-fastest order, N = COUT.  Its
-// input halo -- 3 z planes x (TY + 2) rows x the brick's x range, both
-// 8-channel halves -- is staged once by bulk-tensor copies that fill zeros
-// outside the grid (the convolution's zero padding), each half in its own
-// "chunk plane" so that 8 consecutive x voxels form one 128-byte core matrix
-// of the no-swizzle K-major layout.  Every tap's A operand is then a window
-// of that plane: the descriptor's start moves by (dz, dy) rows and, with TY = 1
-// (one 130-voxel row), by dx voxels; with TY > 1 the rows of the window must
-// be TX apart, so three copies shifted by dx = -1, 0, 1 are staged instead.
-// All 27 taps' weights sit in shared memory as B operands; one thread issues
-// the 27 MMAs (K = 16 each) back to back and commits them to an mbarrier.
-// No per-tap gather and no per-tap block barrier: the 16-channel layers (the
-// finest level of the U-Net) were latency-bound on exactly those.
-template <int COUT, int TX>
-struct RowTile {
-    static constexpr int TY = 128 / TX;
-    static constexpr bool SHIFT = TY > 1;
-    static constexpr int BOXX = SHIFT ? TX : TX + 2;       // x extent of one staged box
-    static constexpr int NSH = SHIFT ? 3 : 1;              // staged dx copies
-    static constexpr int ROWS = 3 * (TY + 2);               // (z, y) rows of a box
-    static constexpr int CH = ROWS * BOXX * 16;             // bytes of one box (8 channels)
-    static constexpr int CHP = (CH + 127) / 128 * 128;      // its slot (128-byte aligned)
-    static constexpr int ABYTES = NSH * 2 * CHP;
-    static constexpr int BBYTES = 27 * 2 * COUT * 16;
-    static constexpr int SMEM = ABYTES + BBYTES + 1024;
-    static_assert(TX % 8 == 0 && TX * TY == 128, "a brick is 128 voxels, whole core matrices in x");
-    static_assert(SMEM <= 200 * 1024, "row conv stage exceeds the shared allocation");
+// Weight gradient: gw[co][t][ci] += sum_v x[v + d_t][ci] gy[v][co].  K = voxels: a
+// brick is 8 MMAs of K = 16 (two of its rows), both operands MN-major (8 channels
+// of a voxel are 16 contiguous bytes, 8 voxels of a row one core matrix), so
+// neither is gathered or transposed.  The chunks of the halo's three planes are M
+// together (3 Cin rows: three taps in one MMA; Cin = 64 takes two MMAs; rows past
+// the last chunk read what lies behind it in shared memory and are never looked
+// at), N = Cout, and the nine (q, x) offsets are nine windows with sums of their
+// own in TMEM, dealt over blockIdx.y where they exceed it.  A CTA (one per SM: it
+// takes all of TMEM) walks its bricks with two buffers; every WG_FLUSH bricks (2048
+// voxels, so that the FP32 sums in TMEM stay short) it adds its sums to gw.
+// Measured against per-element gathers: 48x40x32, 16 -> 16 channels 284 -> 15 us;
+// 24x20x16, 16 -> 32 273 -> 7 us; 12x10x8, 64 -> 32 131 -> 10 us.
+constexpr int WG_FLUSH = 16;
+template <int CIN, int COUT>
+struct WgTile {
+    static constexpr int CH = CIN / 8;
+    static constexpr int MP = (3 * CIN + 127) / 128;                   // MMAs over M
+    static constexpr int WIN = MP * COUT <= 56 ? 9 : (MP * COUT == 64 ? 5 : 3);   // windows of a CTA
+    static constexpr int GROUPS = (9 + WIN - 1) / WIN;
+    static constexpr int XB = 3 * CH * PLB, GB = (COUT / 8) * GPB;
+    static constexpr int ALL = 2 * (GB + XB);
+    static constexpr int REACH = 2 * GB + XB + MP * 16 * PLB;          // (the second buffer's last row)
+    static constexpr int SMEM = (ALL > REACH ? ALL : REACH) + 1024;
+    static_assert(WIN * MP * COUT <= 512 && SMEM <= 226 * 1024, "wgrad exceeds TMEM or shared memory");
 };
-
-struct RowConvArgs {
-    int nx, ny, nz;
-    const bf16_t* w;
-    const float* bias;
-    bf16_t* out16;
-    float* out32;
-    int relu;
-    int* err;
-};
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-        : "memory");
-}
-
-template <int COUT, int TX>
-__global__ void __launch_bounds__(CT) k_conv3d_row(RowConvArgs a, const __grid_constant__ CUtensorMap in_map) {
-    using T = RowTile<COUT, TX>;
-    extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t bar[2];   // 0: the input halo landed; 1: the MMAs finished
-    __shared__ uint32_t tmem_sh;
-    constexpr uint32_t NCOL = 32;
-    constexpr uint32_t IDESC = idesc_bf16(128, COUT);
-    static_assert(COUT == 16 || COUT == 32, "row conv: N = 16 or 32");
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int ntx = a.nx / TX, nty = a.ny / T::TY;
-    const int bx = blockIdx.x % ntx, by = (blockIdx.x / ntx) % nty, bz = blockIdx.x / (ntx * nty);
-    const int x0 = bx * TX, y0 = by * T::TY, z0 = bz;
-    unsigned char* Bs = sm + T::ABYTES;
-    if (warp == 0) tmem_alloc(&tmem_sh, NCOL);
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        fence_mbar_init();
-    }
-    tc_before();
-    __syncthreads();
-    tc_after();
-    if (tid == 0) {
-        mbar_expect_tx(&bar[0], (uint32_t)(T::NSH * 2 * T::CH));
-        for (int sh = 0; sh < T::NSH; ++sh)
-            for (int c = 0; c < 2; ++c)
-                tma_load_4d(sm + (sh * 2 + c) * T::CHP, &in_map, 8 * c, T::SHIFT ? x0 + sh - 1 : x0 - 1, y0 - 1,
-                            z0 - 1, &bar[0]);
-    }
-    // the 27 taps' weights as B operands: tap t, channel half c, row co
-    for (int q = tid; q < 27 * 2 * COUT; q += CT) {
-        const int t = q / (2 * COUT), r = q - t * (2 * COUT), c = r / COUT, co = r - c * COUT;
-        const uint4 val = reinterpret_cast<const uint4*>(a.w + ((long long)co * 27 + t) * 16)[c];
-        *reinterpret_cast<uint4*>(Bs + t * (2 * COUT * 16) + c * (COUT * 16) + (co >> 3) * 128 + (co & 7) * 16) =
-            val;
-    }
-    fence_async_smem();
-    tc_before();
-    __syncthreads();
-    tc_after();
-    const uint32_t tmem = tmem_sh;
-    const uint32_t sbase = smem_u32(sm);
-    bool ok = true;
-    if (tid == 0) {
-        if (!mbar_wait(&bar[0], 0)) ok = false;
-        tc_after();
-        if (ok) {
-            for (int t = 0; t < 27; ++t) {
-                const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;   // 0..2 (offset + 1)
-                const uint32_t arow = (uint32_t)((dz * (T::TY + 2) + dy) * T::BOXX * 16);
-                const uint32_t aoff = T::SHIFT ? (uint32_t)(dx * 2 * T::CHP) + arow : arow + (uint32_t)(dx * 16);
-                const uint64_t ad = sdesc(sbase + aoff, T::CHP, 128);
-                const uint64_t bd = sdesc(sbase + T::ABYTES + t * (2 * COUT * 16), COUT * 16, 128);
-                mma_bf16(tmem, ad, bd, IDESC, t > 0 ? 1u : 0u);
-            }
-        }
-        mma_commit(&bar[1]);   // arrives when every MMA issued above has finished (or at once)
-    }
-    __syncwarp();
-    if (!mbar_wait(&bar[1], 0)) ok = false;
-    tc_after();
-    const int x = x0 + tid % TX, y = y0 + tid / TX;
-    const long long v = ((long long)z0 * a.ny + y) * a.nx + x;
-#pragma unroll
-    for (int c0 = 0; c0 < COUT; c0 += 16) {
-        float acc[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-        if (ok) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float s = acc[i] + (a.bias ? a.bias[c0 + i] : 0.f);
-                if (a.relu) s = fmaxf(s, 0.f);
-                acc[i] = s;
-            }
-            if (a.out16) {
-                uint4* dst = reinterpret_cast<uint4*>(a.out16 + v * COUT + c0);
-                dst[0] = make_uint4(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]), pack2(acc[4], acc[5]),
-                                    pack2(acc[6], acc[7]));
-                dst[1] = make_uint4(pack2(acc[8], acc[9]), pack2(acc[10], acc[11]), pack2(acc[12], acc[13]),
-                                    pack2(acc[14], acc[15]));
-            } else {
-                float4* dst = reinterpret_cast<float4*>(a.out32 + v * COUT + c0);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    dst[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-            }
-        }
-    }
-    if (!ok) {   // a wait ran out: the copies and MMAs in flight get a second bounded wait
-        mbar_wait(&bar[0], 0);
-        mbar_wait(&bar[1], 0);
-        atomicExch(a.err, 1);
-    }
-    tc_before();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, NCOL);
-}
-
-// Weight gradient: D[r][co] = sum_v x[v + d_t][ci] gy[v][co], r = t*CIN + ci.
-// CTA (blockIdx.x = 128-row tile of r, blockIdx.y = chunk of WG_VOX voxels);
-// stages of 32 voxels (two MMAs of K = 16), FP32 atomics into gw.
-constexpr int WG_VOX = 2048;
-constexpr int WG_STAGE = WG_STAGE_;
 
 struct WgradArgs {
-    int nx, ny, nz, nvox;
     const bf16_t* x;
     const bf16_t* gy;
     float* gw;
+    int bricks;
     int* err;
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT) k_conv3d_wgrad(WgradArgs a) {
+__global__ void __launch_bounds__(CT + 32) k_conv3d_wgrad(WgradArgs a, Brick b) {
+    using T = WgTile<CIN, COUT>;
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar_f[2], bar_e[2], bar_d, bar_r;   // a brick landed / used; sums complete / read
     __shared__ uint32_t tmem_sh;
-    constexpr int AB = 128 * WG_STAGE * 2;    // 128 rows x 32 voxels bf16
-    constexpr int BB = COUT * WG_STAGE * 2;
-    constexpr int SB = AB + BB;
-    static_assert(2 * SB + 1024 == wgrad_smem<CIN, COUT>() && wgrad_smem<CIN, COUT>() <= CONV_SMEM_MAX,
-                  "wgrad stages exceed the shared allocation");
-    constexpr uint32_t NCOL = COUT < 32 ? 32 : COUT;
-    constexpr uint32_t IDESC = idesc_bf16(128, COUT);
-    constexpr int R = 27 * CIN;
+    constexpr uint32_t IDESC = idesc_bf16(128, COUT) | (1u << 15) | (1u << 16);   // A and B MN-major
     const int tid = threadIdx.x, warp = tid >> 5;
-    if (warp == 0) tmem_alloc(&tmem_sh, NCOL);
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+    if (warp == 0) tmem_alloc(&tmem_sh, 512);
+    if (tid == CT) {
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&bar_f[q], CT);
+            mbar_init(&bar_e[q], 1);
+        }
+        mbar_init(&bar_d, 1);
+        mbar_init(&bar_r, CT);
         fence_mbar_init();
     }
     tc_before();
     __syncthreads();
     tc_after();
     const uint32_t tmem = tmem_sh;
-    const uint32_t sbase = smem_u32(sm);
-    const int r = blockIdx.x * CT + tid;
-    const bool rok = r < R;
-    const int t = rok ? r / CIN : 0, ci = rok ? r - (r / CIN) * CIN : 0;
-    const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-    const long long v_begin = (long long)blockIdx.y * WG_VOX;
-    const long long v_end = min((long long)a.nvox, v_begin + WG_VOX);
-    const int nstage = (int)((v_end - v_begin + WG_STAGE - 1) / WG_STAGE);
+    const int w0 = blockIdx.y * T::WIN, nw = min(T::WIN, 9 - w0);
+    const int n = (a.bricks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // its bricks
+    auto flushes = [&](int i) { return i == n - 1 || i % WG_FLUSH == WG_FLUSH - 1; };
     bool ok = true;
-    for (int s = 0; s < nstage; ++s) {
-        const int buf = s & 1;
-        if (s >= 2 && !mbar_wait(&bar[buf], ((s - 2) >> 1) & 1)) ok = false;
-        unsigned char* A = sm + buf * SB;
-        unsigned char* B = A + AB;
-        const long long v0 = v_begin + (long long)s * WG_STAGE;
-        // A row r: x[v + d_t][ci] for the stage's 32 voxels (8 per core-matrix row)
-        int vx = (int)(v0 % a.nx);
-        long long rr = v0 / a.nx;
-        int vy = (int)(rr % a.ny), vz = (int)(rr / a.ny);
+    if (tid < CT) {
+        auto load = [&](int i) {
+            const int buf = i & 1;
+            if (i >= 2 && ok && !mbar_wait(&bar_e[buf], ((i >> 1) - 1) & 1)) ok = false;
+            if (!ok) return;
+            int x0, y0, z0;
+            b.origin((int)blockIdx.x + i * (int)gridDim.x, x0, y0, z0);
+            stage<COUT, 0>(sm + buf * T::GB, a.gy, b, x0, y0, z0, 1, tid);
+            stage<CIN, 1>(sm + 2 * T::GB + buf * T::XB, a.x, b, x0, y0, z0, 3, tid);
+        };
+        load(0);
+        copy_commit();
+        int done = 0;
+        for (int i = 0; i < n; ++i) {
+            if (i + 1 < n) load(i + 1);
+            copy_commit();
+            copy_wait<1>();
+            fence_async_smem();
+            mbar_arrive(&bar_f[i & 1]);
+            if (!flushes(i)) continue;
+            if (ok && !mbar_wait(&bar_d, done & 1)) ok = false;
+            ++done;
+            tc_after();
+            for (int j = 0; j < nw; ++j)
 #pragma unroll
-        for (int c = 0; c < WG_STAGE / 8; ++c) {
-            uint32_t w4[4];
+                for (int m = 0; m < T::MP; ++m) {
+                    if (m * 128 + warp * 32 >= 3 * CIN) continue;
+                    // this lane's row: channel ci of the halo's plane p
+                    const int row = m * 128 + tid, p = row / CIN, ci = row % CIN, q = (w0 + j) / 3, dx = (w0 + j) % 3;
+                    const int t = b.along_z ? q * 9 + p * 3 + dx : p * 9 + q * 3 + dx;
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                float pair[2];
+                    for (int c0 = 0; c0 < COUT; c0 += 16) {
+                        float acc[16];
+                        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((j * T::MP + m) * COUT + c0), acc);
+                        if (row >= 3 * CIN || !ok) continue;
+                        // a warp adds to consecutive floats
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const long long vv = v0 + c * 8 + h * 2 + e;
-                    float val = 0.f;
-                    const int xs = vx + dx, ys = vy + dy, zs = vz + dz;
-                    if (rok && vv < v_end && xs >= 0 && xs < a.nx && ys >= 0 && ys < a.ny && zs >= 0 &&
-                        zs < a.nz)
-                        val = bf2f(a.x[(((long long)zs * a.ny + ys) * a.nx + xs) * CIN + ci]);
-                    pair[e] = val;
-                    if (++vx == a.nx) {
-                        vx = 0;
-                        if (++vy == a.ny) { vy = 0; ++vz; }
+                        for (int e = 0; e < 16; ++e) atomicAdd(&a.gw[((long long)(c0 + e) * 27 + t) * CIN + ci], acc[e]);
                     }
                 }
-                w4[h] = pack2(pair[0], pair[1]);
-            }
-            *reinterpret_cast<uint4*>(A + c * 2048 + (tid >> 3) * 128 + (tid & 7) * 16) =
-                make_uint4(w4[0], w4[1], w4[2], w4[3]);
+            tc_before();
+            mbar_arrive(&bar_r);
         }
-        // B row co: gy[v][co] for the same voxels
-        for (int q = tid; q < COUT * (WG_STAGE / 8); q += CT) {
-            const int co = q % COUT, c = q / COUT;
-            uint32_t w4[4];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const long long va = v0 + c * 8 + h * 2;
-                const float g0 = va < v_end ? bf2f(a.gy[va * COUT + co]) : 0.f;
-                const float g1 = va + 1 < v_end ? bf2f(a.gy[(va + 1) * COUT + co]) : 0.f;
-                w4[h] = pack2(g0, g1);
-            }
-            *reinterpret_cast<uint4*>(B + c * (COUT * 16) + (co >> 3) * 128 + (co & 7) * 16) =
-                make_uint4(w4[0], w4[1], w4[2], w4[3]);
-        }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
+    } else if (tid == CT) {
+        int done = 0;
+        for (int i = 0; i < n; ++i) {
+            const int buf = i & 1;
+            if (ok && i % WG_FLUSH == 0 && i > 0 && !mbar_wait(&bar_r, (done - 1) & 1)) ok = false;
+            if (ok && !mbar_wait(&bar_f[buf], (i >> 1) & 1)) ok = false;
             tc_after();
+            if (ok) {
+                const uint64_t g0 = sdesc(smem_u32(sm) + buf * T::GB, 128, GPB);
+                const uint64_t x0 = sdesc(smem_u32(sm) + 2 * T::GB + buf * T::XB, ROWB, PLB);
+                uint32_t d = tmem;
+#pragma unroll 1
+                for (int j = w0; j < w0 + nw; ++j) {
+                    const uint64_t xw = x0 + (uint32_t)(j / 3 * (ROWB / 16) + j % 3);
+#pragma unroll 1
+                    for (int m = 0; m < T::MP; ++m, d += COUT)
 #pragma unroll
-            for (int kk = 0; kk < WG_STAGE / 16; ++kk) {
-                const uint64_t ad = sdesc(sbase + buf * SB + 2 * kk * 2048, 2048, 128);
-                const uint64_t bd = sdesc(sbase + buf * SB + AB + 2 * kk * (COUT * 16), COUT * 16, 128);
-                mma_bf16(tmem, ad, bd, IDESC, (s > 0 || kk > 0) ? 1u : 0u);
+                        for (int s = 0; s < BK_Q / 2; ++s)   // K groups of 8 voxels: a halo row / 128 bytes apart
+                            mma_bf16(d, xw + (uint32_t)(m * PLB) + 2 * s * (ROWB / 16), g0 + 2 * s * 8, IDESC,
+                                     (i % WG_FLUSH || s) ? 1u : 0u);
+                }
             }
-            mma_commit(&bar[buf]);
+            mma_commit(&bar_e[buf]);
+            if (flushes(i)) {
+                mma_commit(&bar_d);
+                ++done;
+            }
         }
     }
-    const int last = nstage - 1;
-    if (nstage > 0 && !mbar_wait(&bar[last & 1], (last >> 1) & 1)) ok = false;
-    tc_after();
-    if (nstage > 0) {
-#pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
-            float acc[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-            if (rok && ok) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) atomicAdd(&a.gw[(long long)(c0 + i) * R + r], acc[i]);
-            }
-        }
-    }
-    if (!ok) {
-        if (nstage > 0) mbar_wait(&bar[last & 1], (last >> 1) & 1);
+    ok = __syncthreads_and(ok);
+    if (!ok) {   // a wait ran out: the MMAs in flight get a second bounded wait
+        mbar_wait(&bar_e[0], 0);
+        mbar_wait(&bar_e[1], 0);
         if (tid == 0) atomicExch(a.err, 1);
     }
     tc_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, NCOL);
+    if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// gb[co] += sum_v gy[v][co]
-__global__ void k_bias_grad(const bf16_t* __restrict__ gy, int nvox, int cout, float* gb) {
+// gb[co] += sum_v gy[v][co], for the layers of blockIdx.y (a launch each cost
+// 2.7 us, all seven together 6 us).
+struct BiasArgs {
+    const bf16_t* gy[WPF_NET_LAYERS];
+    float* gb[WPF_NET_LAYERS];
+    int nvox[WPF_NET_LAYERS], cout[WPF_NET_LAYERS];
+};
+__global__ void k_bias_grad(BiasArgs a) {
     __shared__ float s[64];
     if (threadIdx.x < 64) s[threadIdx.x] = 0.f;
     __syncthreads();
+    const int l = blockIdx.y, cout = a.cout[l], nvox = a.nvox[l];
+    const bf16_t* __restrict__ gy = a.gy[l];
     const int co = threadIdx.x % cout;
     const int lanes = blockDim.x / cout;
     float acc = 0.f;
@@ -548,7 +568,7 @@ __global__ void k_bias_grad(const bf16_t* __restrict__ gy, int nvox, int cout, f
         acc += bf2f(gy[v * cout + co]);
     atomicAdd(&s[co], acc);
     __syncthreads();
-    if (threadIdx.x < cout) atomicAdd(&gb[threadIdx.x], s[threadIdx.x]);
+    if (threadIdx.x < cout) atomicAdd(&a.gb[l][threadIdx.x], s[threadIdx.x]);
 }
 
 // ---- elementwise pieces of the U-Net ----------------------------------------------
@@ -665,14 +685,8 @@ __global__ void k_loss_sums(const float* __restrict__ out, int cstride, const fl
         s += (double)w * d * d;
         m += w;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_down_sync(0xffffffffu, s, o);
-        m += __shfl_down_sync(0xffffffffu, m, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&acc[0], s);
-        atomicAdd(&acc[1], m);
-    }
+    block_add(s, &acc[0]);   // (one atomic per block: every block adds to the same two words)
+    block_add(m, &acc[1]);
 }
 // g[v][0] = 2 mask (o - t) / sum(mask), g[v][1..C) = 0   (bf16)
 __global__ void k_loss_grad(const float* __restrict__ out, int C, const float* __restrict__ tgt,
@@ -683,8 +697,9 @@ __global__ void k_loss_grad(const float* __restrict__ out, int C, const float* _
          v += (long long)gridDim.x * blockDim.x) {
         const float w = mask ? mask[v] : 1.f;
         const float d = out[v * C] - tgt[v];
-        g[v * C] = f2bf(2.f * w * d * inv);
-        for (int c = 1; c < C; ++c) g[v * C + c] = 0;
+        uint4* o = reinterpret_cast<uint4*>(g + v * C);
+        o[0] = make_uint4((uint32_t)f2bf(2.f * w * d * inv), 0u, 0u, 0u);
+        for (int c = 1; c < C / 8; ++c) o[c] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -703,16 +718,21 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
     }
 }
 
-// bf16 copies of one layer's weights: w16[co][t][ci] and the flipped transpose
-// wt16[ci][26 - t][co] (the weights of the data-gradient convolution).
-__global__ void k_pack_weights(const float* __restrict__ w, int cin, int cout, bf16_t* __restrict__ w16,
-                               bf16_t* __restrict__ wt16) {
+// bf16 copies of the weights of layer blockIdx.y: w16[co][t][ci] and the flipped
+// transpose wt16[ci][26 - t][co] (the weights of the data-gradient convolution).
+struct PackArgs {
+    const float* w[WPF_NET_LAYERS];
+    bf16_t *w16[WPF_NET_LAYERS], *wt16[WPF_NET_LAYERS];
+    int cin[WPF_NET_LAYERS], cout[WPF_NET_LAYERS];
+};
+__global__ void k_pack_weights(PackArgs a) {
+    const int l = blockIdx.y, cin = a.cin[l], cout = a.cout[l];
     const int n = cout * 27 * cin;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int ci = q % cin, t = (q / cin) % 27, co = q / (27 * cin);
-        const bf16_t b = f2bf(w[q]);
-        w16[q] = b;
-        wt16[((long long)ci * 27 + (26 - t)) * cout + co] = b;
+        const bf16_t b = f2bf(a.w[l][q]);
+        a.w16[l][q] = b;
+        a.wt16[l][((long long)ci * 27 + (26 - t)) * cout + co] = b;
     }
 }
 
@@ -736,66 +756,20 @@ static const int LAYER_LEVEL[WPF_NET_LAYERS] = {0, 1, 2, 3, 2, 1, 0};
 
 template <int CIN, int COUT>
 static int launch_conv_t(const ConvArgs& a, cudaStream_t s) {
+    using T = ConvTile<CIN, COUT>;
     static bool attr = false;
     if (!attr) {
-        WPF_CUDA(cudaFuncSetAttribute(k_conv3d<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      conv_smem<CIN, COUT>()));
+        WPF_CUDA(cudaFuncSetAttribute(k_conv3d_tile<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      T::smem(T::MOST)));
         attr = true;
     }
-    const unsigned grid = (unsigned)((a.nvox + CT - 1) / CT);
-    k_conv3d<CIN, COUT><<<grid, CT, conv_smem<CIN, COUT>(), s>>>(a);
+    const Brick b = make_brick(a.nx, a.ny, a.nz, T::MOST, sm_count());
+    k_conv3d_tile<CIN, COUT><<<(unsigned)b.count(), CT + 32, T::smem(b.nb), s>>>(a, b);
     WPF_CUDA(cudaGetLastError());
-    return WPF_OK;
-}
-
-// The row-tiled kernel on its brick grid; WPF_ERR_CUDA when the tensor map
-// cannot be encoded (the caller then uses the gather kernel).
-template <int COUT, int TX>
-static int launch_conv_row(const ConvArgs& a, cudaStream_t s) {
-    using T = RowTile<COUT, TX>;
-    static bool attr = false;
-    if (!attr) {
-        WPF_CUDA(cudaFuncSetAttribute(k_conv3d_row<COUT, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      T::SMEM));
-        attr = true;
-    }
-    const EncodeTiledFn f = tensor_map_encoder();
-    if (!f) return WPF_ERR_CUDA;
-    CUtensorMap m;
-    const cuuint64_t dims[4] = {16, (cuuint64_t)a.nx, (cuuint64_t)a.ny, (cuuint64_t)a.nz};
-    const cuuint64_t strides[3] = {32, (cuuint64_t)a.nx * 32, (cuuint64_t)a.nx * a.ny * 32};
-    const cuuint32_t box[4] = {8, (cuuint32_t)T::BOXX, (cuuint32_t)(T::TY + 2), 3};
-    const cuuint32_t es[4] = {1, 1, 1, 1};
-    if (f(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)a.in, dims, strides, box, es,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return WPF_ERR_CUDA;
-    RowConvArgs r;
-    r.nx = a.nx; r.ny = a.ny; r.nz = a.nz;
-    r.w = a.w; r.bias = a.bias; r.out16 = a.out16; r.out32 = a.out32; r.relu = a.relu; r.err = a.err;
-    const unsigned grid = (unsigned)((a.nx / TX) * (a.ny / T::TY) * a.nz);
-    k_conv3d_row<COUT, TX><<<grid, CT, T::SMEM, s>>>(r, m);
-    WPF_CUDA(cudaGetLastError());
-    return WPF_OK;
-}
-
-template <int COUT>
-static int try_conv_row(const ConvArgs& a, cudaStream_t s, bool* done) {
-    *done = true;
-#define WPF_ROW_CASE(TX) \
-    if (a.nx % TX == 0 && a.ny % (128 / TX) == 0) return launch_conv_row<COUT, TX>(a, s);
-    WPF_ROW_CASE(128) WPF_ROW_CASE(64) WPF_ROW_CASE(32) WPF_ROW_CASE(16)
-#undef WPF_ROW_CASE
-    *done = false;
     return WPF_OK;
 }
 
 static int launch_conv(int cin, int cout, const ConvArgs& a, cudaStream_t s) {
-    if (cin == 16 && (cout == 16 || cout == 32) && (long long)a.nx * a.ny * a.nz == a.nvox) {
-        bool done = false;
-        const int rc = cout == 16 ? try_conv_row<16>(a, s, &done) : try_conv_row<32>(a, s, &done);
-        if (done) return rc;
-    }
 #define WPF_CONV_CASE(I, O) \
     if (cin == I && cout == O) return launch_conv_t<I, O>(a, s);
     WPF_CONV_CASE(16, 16) WPF_CONV_CASE(16, 32) WPF_CONV_CASE(32, 64) WPF_CONV_CASE(64, 64)
@@ -805,22 +779,29 @@ static int launch_conv(int cin, int cout, const ConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int COUT>
-static int launch_wgrad_t(const WgradArgs& a, cudaStream_t s) {
+static int launch_wgrad_t(int nx, int ny, int nz, const bf16_t* x, const bf16_t* gy, float* gw, int* err,
+                          cudaStream_t s) {
+    using T = WgTile<CIN, COUT>;
     static bool attr = false;
     if (!attr) {
-        WPF_CUDA(cudaFuncSetAttribute(k_conv3d_wgrad<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      wgrad_smem<CIN, COUT>()));
+        WPF_CUDA(cudaFuncSetAttribute(k_conv3d_wgrad<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
         attr = true;
     }
-    const dim3 grid((27 * CIN + CT - 1) / CT, (unsigned)((a.nvox + WG_VOX - 1) / WG_VOX));
-    k_conv3d_wgrad<CIN, COUT><<<grid, CT, wgrad_smem<CIN, COUT>(), s>>>(a);
+    const Brick b = make_brick(nx, ny, nz, 1, 1);
+    WgradArgs a;
+    a.x = x; a.gy = gy; a.gw = gw; a.err = err;
+    a.bricks = b.count();
+    const int split = sm_count() / T::GROUPS > 0 ? sm_count() / T::GROUPS : 1;
+    const dim3 grid((unsigned)(a.bricks < split ? a.bricks : split), T::GROUPS);
+    k_conv3d_wgrad<CIN, COUT><<<grid, CT + 32, T::SMEM, s>>>(a, b);
     WPF_CUDA(cudaGetLastError());
     return WPF_OK;
 }
 
-static int launch_wgrad(int cin, int cout, const WgradArgs& a, cudaStream_t s) {
+static int launch_wgrad(int cin, int cout, int nx, int ny, int nz, const bf16_t* x, const bf16_t* gy, float* gw, int* err,
+                        cudaStream_t s) {
 #define WPF_WG_CASE(I, O) \
-    if (cin == I && cout == O) return launch_wgrad_t<I, O>(a, s);
+    if (cin == I && cout == O) return launch_wgrad_t<I, O>(nx, ny, nz, x, gy, gw, err, s);
     WPF_WG_CASE(16, 16) WPF_WG_CASE(16, 32) WPF_WG_CASE(32, 64) WPF_WG_CASE(64, 64)
     WPF_WG_CASE(64, 32) WPF_WG_CASE(32, 16)
 #undef WPF_WG_CASE
@@ -887,11 +868,16 @@ int conv(wpf_net* n, int l, const bf16_t* in, const bf16_t* w, int cin, int cout
 }
 
 int pack_all(wpf_net* n, cudaStream_t s) {
+    PackArgs a;
     for (int l = 0; l < WPF_NET_LAYERS; ++l) {
         const Layer& L = n->L[l];
-        k_pack_weights<<<ew_grid((long long)L.cout * 27 * L.cin), 256, 0, s>>>(n->p + L.woff, L.cin, L.cout,
-                                                                            L.w16, L.wt16);
+        a.w[l] = n->p + L.woff;
+        a.w16[l] = L.w16;
+        a.wt16[l] = L.wt16;
+        a.cin[l] = L.cin;
+        a.cout[l] = L.cout;
     }
+    k_pack_weights<<<dim3(108, WPF_NET_LAYERS), 256, 0, s>>>(a);   // (64 x 27 x 64: four weights a thread)
     WPF_CUDA(cudaGetLastError());
     return WPF_OK;
 }
@@ -921,14 +907,8 @@ int forward(wpf_net* n, const bf16_t* x, cudaStream_t s) {
 int wgrad(wpf_net* n, int l, const bf16_t* x, const bf16_t* gy, cudaStream_t s) {
     const Layer& L = n->L[l];
     const int lv = L.level;
-    WgradArgs a;
-    a.nx = n->nx[lv]; a.ny = n->ny[lv]; a.nz = n->nz[lv]; a.nvox = (int)n->nvox[lv];
-    a.x = x; a.gy = gy; a.gw = n->g + L.woff; a.err = n->derr;
-    int rc = launch_wgrad(L.cin, L.cout, a, s);
-    if (rc) return rc;
-    k_bias_grad<<<256, 256, 0, s>>>(gy, (int)n->nvox[lv], L.cout, n->g + L.boff);
-    WPF_CUDA(cudaGetLastError());
-    return WPF_OK;
+    int rc = launch_wgrad(L.cin, L.cout, n->nx[lv], n->ny[lv], n->nz[lv], x, gy, n->g + L.woff, n->derr, s);
+    return rc;
 }
 
 int backward(wpf_net* n, const bf16_t* x, cudaStream_t s) {
@@ -963,6 +943,14 @@ int backward(wpf_net* n, const bf16_t* x, cudaStream_t s) {
     k_bwd_pool_skip_relu<<<ew_grid(n->nvox[0] * 16), 256, 0, s>>>(n->gp0, n->gs0, n->y[0], n->gpre[0], X[0], Y[0],
                                                                  Z[0], 16);
     if ((rc = wgrad(n, 0, x, n->gpre[0], s))) return rc;
+    BiasArgs ba;
+    for (int l = 0; l < WPF_NET_LAYERS; ++l) {
+        ba.gy[l] = l == WPF_NET_LAYERS - 1 ? n->gout : n->gpre[l];
+        ba.gb[l] = n->g + n->L[l].boff;
+        ba.nvox[l] = (int)n->nvox[n->L[l].level];
+        ba.cout[l] = n->L[l].cout;
+    }
+    k_bias_grad<<<dim3(256, WPF_NET_LAYERS), 256, 0, s>>>(ba);
     WPF_CUDA(cudaGetLastError());
     return WPF_OK;
 }
@@ -1152,12 +1140,16 @@ int wpf_conv3d_wgrad(int32_t cin, int32_t cout, int32_t nx, int32_t ny, int32_t 
         WPF_CUDA(cudaMalloc((void**)&derr, sizeof(int)));
         WPF_CUDA(cudaMemset(derr, 0, sizeof(int)));
     }
-    WgradArgs a;
-    a.nx = nx; a.ny = ny; a.nz = nz; a.nvox = nx * ny * nz;
-    a.x = x; a.gy = gy; a.gw = gw; a.err = derr;
-    int rc = launch_wgrad(cin, cout, a, s);
+    int rc = launch_wgrad(cin, cout, nx, ny, nz, x, gy, gw, derr, s);
     if (rc) return rc;
-    if (gb) k_bias_grad<<<256, 256, 0, s>>>(gy, nx * ny * nz, cout, gb);
+    if (gb) {
+        BiasArgs ba = {};
+        ba.gy[0] = gy;
+        ba.gb[0] = gb;
+        ba.nvox[0] = nx * ny * nz;
+        ba.cout[0] = cout;
+        k_bias_grad<<<256, 256, 0, s>>>(ba);
+    }
     WPF_CUDA(cudaGetLastError());
     int e = 0;
     WPF_CUDA(cudaMemcpyAsync(&e, derr, sizeof(int), cudaMemcpyDeviceToHost, s));
