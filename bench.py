@@ -471,7 +471,8 @@ def roofline_window(args, arms):
     # cx, cy, cz (12 B), 1/diag (4 B), b (4 B) and the input x (4 B) and
     # writes the output x (4 B): 28 B; the zero-guess first sweep of a cycle
     # reads no x: 24 B; nu = 2 sweeps per side, four per cycle.  Smaller finest
-    # levels run two half-sweep kernels: 20 B per cell each, 12 B zero-guess.
+    # levels run one kernel per half-sweep, 20 B per cell each, the zero-guess
+    # pair in one: 24 B.
     nu = args.nu
     cnt = int(kcnt[KC_SMOOTH0])
     smooth_ms = float(kms[KC_SMOOTH0])
@@ -480,8 +481,8 @@ def roofline_window(args, arms):
         smooth_bytes = (cycles * 24.0 + (cnt - cycles) * 28.0) * ncell
         kname, per_cell = "k_sweep_async<float> (finest level)", 28
     else:
-        n_first = cnt // (4 * nu)
-        smooth_bytes = (n_first * 12.0 + (cnt - n_first) * 20.0) * ncell
+        n_first = cnt // (4 * nu - 1)
+        smooth_bytes = (n_first * 24.0 + (cnt - n_first) * 20.0) * ncell
         kname, per_cell = "k_rbgs<float> (finest level)", 20
     peak, peak_kind = measured_peaks()
     achieved = smooth_bytes / (smooth_ms / 1000.0) / 1e9 if smooth_ms > 0 else None

@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(coarse_nt<R>()) k_coarse(const __grid_constant
             owner[q >> 1][q & 1] = (unsigned char)slab_owner(L.shift, a.ncd, C, min(q, L.nc - 1));
     }
     __syncthreads();
+    pdl_wait();   // the set-up above may run beside the launch before
     {   // the operators: one index space over the levels (both colours of a row in
         // turn), UN slots' loads in flight per thread
         constexpr int UN = 16 / (int)sizeof(R);

@@ -372,6 +372,12 @@ void timer_flush(wpf_handle* h);   // after a synchronisation: fold finished pai
 
 namespace wpf {
 
+// ---- programmatic launches --------------------------------------------------
+// wait: until the launch before is complete and its writes are visible;
+// release: let the launch after start (both do nothing in an ordinary launch).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- error helpers --------------------------------------------------------
 #define WPF_CUDA(call)                                   \
     do {                                                 \

@@ -544,7 +544,7 @@ __global__ void k_coarsen(Grid f, Grid c, const R* __restrict__ fcx, const R* __
 
 template <typename R>
 __device__ __forceinline__ R offsum(const R* __restrict__ cx, const R* __restrict__ cy,
-                                    const R* __restrict__ cz, const R* __restrict__ x, long long n,
+                                    const R* __restrict__ cz, const R* x, long long n,
                                     long long sy, long long sz) {
     return cx[n] * x[n + 1] + cx[n - 1] * x[n - 1] + cy[n] * x[n + sy] + cy[n - sy] * x[n - sy] +
            cz[n] * x[n + sz] + cz[n - sz] * x[n - sz];
@@ -898,31 +898,162 @@ __global__ void __launch_bounds__(SX * SY) k_sweep_async(Grid g, const R* __rest
 template <typename R>
 constexpr size_t sweep_smem() { return sizeof(SweepSlot<R>) * NSLOT + 128; }
 
-// One colour of red-black Gauss-Seidel in place (mid-size levels).  Thread
-// (t,j,k) handles the cell of colour `color` at i = 1 + 2t + ((color+1+j+k) & 1).
+// ---------------------------------------------------------------------------
+// Half-sweeps of the levels between the pipelined sweeps' and the cluster's.
+// Such a level lies in L2 and a launch on it takes 2-6 us, of which about one is
+// the boundary between two launches.  So (a) the launches are as few as the
+// dependences allow: the zero-guess red half-sweep is formed inside the first
+// black one, the coarse correction inside the first black one after it, r.z
+// inside the last red one; (b) each is launched programmatically behind the
+// one before it: it loads what that one does not write (the operator, and
+// arrays that an earlier launch wrote: a launch releases its successor only
+// after its own wait, when everything before it is complete) and then waits.
+// Per half-sweep, boundary included, plain -> programmatic: 36x28x21 1.44 ->
+// 1.05 us, 64^3 2.05 -> 1.79, 100x90x110 3.89 -> 3.31, 128^3 5.76 -> 5.20.
+// Ten launches a level and cycle (nu = 2) became eight: a step of 96x80x72 in
+// FP64 (11 cycles) 4.3 -> 3.75 ms, of 128^3 in FP32 (2 cycles) 747 -> 717 us.
+// Arrays written by the launch before are passed without __restrict__: their
+// loads stay behind the wait.
+// ---------------------------------------------------------------------------
+// The six couplings of a cell; off() sums in offsum's order.
 template <typename R>
-__global__ void k_rbgs(Grid g, const R* __restrict__ cx, const R* __restrict__ cy,
-                       const R* __restrict__ cz, const R* __restrict__ idiag, R* __restrict__ x,
-                       const R* __restrict__ b, int color) {
+struct Links {
+    R xp, xm, yp, ym, zp, zm;
+    __device__ __forceinline__ void load(const R* __restrict__ cx, const R* __restrict__ cy,
+                                         const R* __restrict__ cz, long long n, long long sy, long long sz) {
+        xp = cx[n];
+        xm = cx[n - 1];
+        yp = cy[n];
+        ym = cy[n - sy];
+        zp = cz[n];
+        zm = cz[n - sz];
+    }
+    template <typename F>
+    __device__ __forceinline__ R off(F&& x, long long n, long long sy, long long sz) const {
+        return xp * x(n + 1) + xm * x(n - 1) + yp * x(n + sy) + ym * x(n - sy) + zp * x(n + sz) + zm * x(n - sz);
+    }
+};
+
+// One colour of red-black Gauss-Seidel in place.  Thread (t,j,k) handles the
+// cell of colour `color` (0 red: i+j+k even) at i = 1 + 2t + ((color+1+j+k) & 1).
+template <typename R>
+__global__ void __launch_bounds__(256) k_rbgs(Grid g, const R* __restrict__ cx, const R* __restrict__ cy,
+                                              const R* __restrict__ cz, const R* __restrict__ idiag, R* x,
+                                              const R* __restrict__ b, int color) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int k = 1 + blockIdx.z * blockDim.z + threadIdx.z;
     const int i = 1 + 2 * t + ((color + 1 + j + k) & 1);
-    if (i > g.nx || j > g.ny || k > g.nz) return;
+    const bool on = i <= g.nx && j <= g.ny && k <= g.nz;
     const long long n = g.at(i, j, k);
-    x[n] = idiag[n] * (b[n] + offsum(cx, cy, cz, x, n, g.P, g.S));
+    Links<R> c;
+    R id, rhs;
+    if (on) {
+        c.load(cx, cy, cz, n, g.P, g.S);
+        id = idiag[n];
+        rhs = b[n];
+    }
+    pdl_wait();
+    pdl_release();
+    if (on) x[n] = id * (rhs + c.off([&](long long m) { return x[m]; }, n, g.P, g.S));
 }
 
-// First red sweep from a zero initial guess: red cells get idiag*b, black 0.
+// The last red half-sweep of the cycle on the finest level, with r.z (b = r,
+// x = z): the thread adds its red cell's term and its row partner's, which is
+// one of the neighbours it has read.  A bounded grid walks z, so that the
+// blocks' atomics on one address stay few.  (A separate dot read both arrays
+// again: 4.5 us at 100x90x110.)
 template <typename R>
-__global__ void k_rbgs_first(Grid g, const R* __restrict__ idiag, R* __restrict__ x,
-                             const R* __restrict__ b) {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_rbgs_dot(Grid g, const R* __restrict__ cx, const R* __restrict__ cy,
+                                                  const R* __restrict__ cz, const R* __restrict__ idiag, R* x,
+                                                  const R* __restrict__ b, double* acc) {
+    pdl_wait();
+    pdl_release();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    R d = 0;
+    if (j <= g.ny)
+        for (int k = 1 + blockIdx.z * blockDim.z + threadIdx.z; k <= g.nz; k += gridDim.z * blockDim.z) {
+            const int e = (1 + j + k) & 1;
+            const int i = 1 + 2 * t + e, ip = 2 + 2 * t - e;   // the red cell and its black partner
+            const long long n = g.at(i, j, k), np = n + ip - i;
+            if (ip <= g.nx) d += b[np] * x[np];
+            if (i <= g.nx) {
+                Links<R> c;
+                c.load(cx, cy, cz, n, g.P, g.S);
+                const R rhs = b[n];
+                const R v = idiag[n] * (rhs + c.off([&](long long m) { return x[m]; }, n, g.P, g.S));
+                x[n] = v;
+                d += rhs * v;
+            }
+        }
+    block_add(d, acc);
+}
+
+// The first red and black half-sweeps from a zero guess: red cells are
+// idiag*b, and a black cell forms its six red neighbours from idiag and b
+// itself (the same products).  Thread (t,j,k) writes the row pair 2t+1, 2t+2.
+// (b: the launch before may have written it.)
+template <typename R>
+__global__ void __launch_bounds__(256) k_rbgs_zero(Grid g, const R* __restrict__ cx, const R* __restrict__ cy,
+                                                   const R* __restrict__ cz, const R* __restrict__ idiag,
+                                                   R* x, const R* b) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int k = 1 + blockIdx.z * blockDim.z + threadIdx.z;
-    if (i > g.nx || j > g.ny || k > g.nz) return;
+    const int e = (j + k) & 1;
+    const int i = 1 + 2 * t + e, ir = 2 + 2 * t - e;   // the black cell and its red partner
+    const bool row = j <= g.ny && k <= g.nz, on = row && i <= g.nx;
+    const long long n = g.at(i, j, k), nr = n + ir - i;
+    Links<R> c, d;   // couplings; the neighbours' idiag
+    R id;
+    if (on) {
+        c.load(cx, cy, cz, n, g.P, g.S);
+        id = idiag[n];
+        d = {idiag[n + 1], idiag[n - 1], idiag[n + g.P], idiag[n - g.P], idiag[n + g.S], idiag[n - g.S]};
+    }
+    pdl_wait();
+    pdl_release();
+    if (row && ir <= g.nx) x[nr] = idiag[nr] * b[nr];
+    if (on)
+        x[n] = id * (b[n] + (c.xp * (d.xp * b[n + 1]) + c.xm * (d.xm * b[n - 1]) + c.yp * (d.yp * b[n + g.P]) +
+                             c.ym * (d.ym * b[n - g.P]) + c.zp * (d.zp * b[n + g.S]) + c.zm * (d.zm * b[n - g.S])));
+}
+
+// The first black half-sweep after the coarse correction x += x_c(parent) of
+// the live cells.  Only the red cells' corrected values are ever read (this
+// half-sweep replaces the black ones, the next one the red ones), so they are
+// formed here and not written.  (xc: written by the launch before.)
+template <typename R>
+__global__ void __launch_bounds__(256) k_rbgs_corr(Grid g, Grid gc, const R* __restrict__ cx, const R* __restrict__ cy,
+                                                   const R* __restrict__ cz, const R* __restrict__ idiag, R* x,
+                                                   const R* __restrict__ b, const R* xc) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = 1 + blockIdx.z * blockDim.z + threadIdx.z;
+    const int i = 1 + 2 * t + ((j + k) & 1);
+    const bool on = i <= g.nx && j <= g.ny && k <= g.nz;
     const long long n = g.at(i, j, k);
-    x[n] = ((i + j + k) & 1) ? (R)0 : idiag[n] * b[n];
+    Links<R> c, d, v;   // couplings; the neighbours' idiag and x
+    R id, rhs;
+    if (on) {
+        c.load(cx, cy, cz, n, g.P, g.S);
+        id = idiag[n];
+        rhs = b[n];
+        d = {idiag[n + 1], idiag[n - 1], idiag[n + g.P], idiag[n - g.P], idiag[n + g.S], idiag[n - g.S]};
+        v = {x[n + 1], x[n - 1], x[n + g.P], x[n - g.P], x[n + g.S], x[n - g.S]};
+    }
+    pdl_wait();
+    pdl_release();
+    if (!on) return;
+    auto parent = [&](int di, int dj, int dk) { return xc[gc.at((i + di + 1) >> 1, (j + dj + 1) >> 1, (k + dk + 1) >> 1)]; };
+    if (d.xp != (R)0) v.xp += parent(1, 0, 0);
+    if (d.xm != (R)0) v.xm += parent(-1, 0, 0);
+    if (d.yp != (R)0) v.yp += parent(0, 1, 0);
+    if (d.ym != (R)0) v.ym += parent(0, -1, 0);
+    if (d.zp != (R)0) v.zp += parent(0, 0, 1);
+    if (d.zm != (R)0) v.zm += parent(0, 0, -1);
+    x[n] = id * (rhs + (c.xp * v.xp + c.xm * v.xm + c.yp * v.yp + c.ym * v.ym + c.zp * v.zp + c.zm * v.zm));
 }
 
 // x_l += x_{l+1}(parent) on live cells, four cells of a row per thread:
@@ -972,32 +1103,50 @@ static void launch_prolong(wpf_handle* h, const Grid& f, const Grid& c, const R*
     WPF_LAUNCH(h, KC_MGREST, k_prolong4<R><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(f, c, idiag, x, xc));
 }
 
-// Residual of level l restricted (summed over the aggregate) into b of level l+1.
+// Residual of level l restricted (summed over the aggregate) into b of level
+// l+1, after a black half-sweep: a live black cell's residual is zero then, so
+// the four red cells of an aggregate are summed, and a black one only where it
+// is dead (its couplings, if it has any, meet x = 0 there).  Summing all eight
+// took twice the loads for the rounding of zero.
+// (x: written by the launch before.)
 template <typename R>
-__global__ void k_resid_restrict(Grid f, Grid c, const R* __restrict__ cx, const R* __restrict__ cy,
-                                 const R* __restrict__ cz, const R* __restrict__ diag,
-                                 const R* __restrict__ x, const R* __restrict__ b,
-                                 R* __restrict__ bc) {
+__global__ void __launch_bounds__(256) k_resid_restrict(Grid f, Grid c, const R* __restrict__ cx,
+                                                        const R* __restrict__ cy, const R* __restrict__ cz,
+                                                        const R* __restrict__ diag, const R* __restrict__ idiag,
+                                                        const R* x, const R* __restrict__ b, R* __restrict__ bc) {
     const int I = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int J = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int K = 1 + blockIdx.z * blockDim.z + threadIdx.z;
-    if (I > c.nx || J > c.ny || K > c.nz) return;
-    R s = 0;
-    for (int dk = 0; dk < 2; ++dk) {
-        const int k = 2 * K - 1 + dk;
-        if (k > f.nz) break;
-        for (int dj = 0; dj < 2; ++dj) {
-            const int j = 2 * J - 1 + dj;
-            if (j > f.ny) break;
-            for (int di = 0; di < 2; ++di) {
-                const int i = 2 * I - 1 + di;
-                if (i > f.nx) break;
-                const long long n = f.at(i, j, k);
-                s += b[n] - (diag[n] * x[n] - offsum(cx, cy, cz, x, n, f.P, f.S));
-            }
+    const bool on = I <= c.nx && J <= c.ny && K <= c.nz;
+    const long long n0 = f.at(2 * I - 1, 2 * J - 1, 2 * K - 1);   // i+j+k odd: black
+    const bool ex = 2 * I <= f.nx, ey = 2 * J <= f.ny, ez = 2 * K <= f.nz;
+    const long long red[4] = {n0 + 1, n0 + f.P, n0 + f.S, n0 + f.S + f.P + 1};
+    const bool red_on[4] = {on && ex, on && ey, on && ez, on && ex && ey && ez};
+    const long long blk[4] = {n0, n0 + f.P + 1, n0 + f.S + 1, n0 + f.S + f.P};
+    const bool blk_on[4] = {on, on && ex && ey, on && ex && ez, on && ey && ez};
+    Links<R> l[4];
+    R dg[4], rhs[4];
+    bool dead[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (red_on[q]) {
+            l[q].load(cx, cy, cz, red[q], f.P, f.S);
+            dg[q] = diag[red[q]];
+            rhs[q] = b[red[q]];
         }
+        dead[q] = blk_on[q] && idiag[blk[q]] == (R)0;
     }
-    bc[c.at(I, J, K)] = s;
+    pdl_wait();
+    pdl_release();
+    auto xv = [&](long long m) { return x[m]; };
+    R s = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (red_on[q]) s += rhs[q] - (dg[q] * x[red[q]] - l[q].off(xv, red[q], f.P, f.S));
+    if (dead[0] || dead[1] || dead[2] || dead[3])
+        for (int q = 0; q < 4; ++q)
+            if (dead[q]) s += b[blk[q]] - (diag[blk[q]] * x[blk[q]] - offsum(cx, cy, cz, x, blk[q], f.P, f.S));
+    if (on) bc[c.at(I, J, K)] = s;
 }
 
 // ---- PCG vector kernels (persistent row loops, one atomic per block) -------
@@ -1267,15 +1416,14 @@ static long long ncells(const Grid& g) { return (long long)g.nx * g.ny * g.nz; }
 constexpr long long BIG_CELLS = 1LL << 23;   // default: levels swept by the pipelined kernel
 
 // One preconditioner cycle z = M r (level 0 aliases b = r, x = z); rz != null
-// accumulates r.z (in the last level-0 sweep when that level is a big one,
-// else by a dot).  Level l recurses gamma(l) times (gamma = 2 from level
-// opts.w_from_level on: a W-cycle on the mid levels; 1 above: a V-cycle),
-// with symmetric smoothing around each coarse correction, so the cycle stays
-// a symmetric preconditioner.  Big levels sweep between their two buffers so
-// that the 2*nu sweeps end in the level's output buffer x (the first
-// pre-sweep writes xs, the last post-sweep writes x); mid levels sweep x in
-// place; the levels that fit a cluster's shared memory run in one k_coarse launch
-// (wpf_coarse.cuh).
+// accumulates r.z in the last sweep on level 0.  Level l recurses gamma(l)
+// times (gamma = 2 from level opts.w_from_level on: a W-cycle on the mid
+// levels; 1 above: a V-cycle), with symmetric smoothing around each coarse
+// correction, so the cycle stays a symmetric preconditioner.  Big levels sweep
+// between their two buffers so that the 2*nu sweeps end in the level's output
+// buffer x (the first pre-sweep writes xs, the last post-sweep writes x); mid
+// levels sweep x in place (k_rbgs and its relatives); the levels that fit a
+// cluster's shared memory run in one k_coarse launch (wpf_coarse.cuh).
 // ---- bulk-tensor maps of the sweep -------------------------------------------------
 EncodeTiledFn tensor_map_encoder() {
     static EncodeTiledFn fn = nullptr;
@@ -1429,8 +1577,25 @@ static CoarsePlan<R> coarse_plan(const wpf_handle* h, const Hierarchy<R>& H, int
     return p;
 }
 
+// Launch k programmatically behind the launch before it on s (see k_rbgs); as an
+// ordinary launch where that one is not a kernel of this cycle, or where the
+// timers put event records between the two.
+template <typename... P, typename... A>
+static cudaError_t launch_behind(bool behind, void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 template <typename R>
-static void launch_coarse(wpf_handle* h, CoarsePlan<R>& p, int cls, double* dot, cudaStream_t s) {
+static void launch_coarse(wpf_handle* h, CoarsePlan<R>& p, int cls, double* dot, bool behind, cudaStream_t s) {
     p.args.dot = dot;
     p.args.err = reinterpret_cast<int*>(h->dsc + S_KERR);
     cudaLaunchConfig_t cfg = {};
@@ -1438,24 +1603,25 @@ static void launch_coarse(wpf_handle* h, CoarsePlan<R>& p, int cls, double* dot,
     cfg.blockDim = dim3(coarse_nt<R>());
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = s;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)p.args.C;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)p.args.C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = behind ? 2 : 1;
     WPF_LAUNCH(h, cls, cudaLaunchKernelEx(&cfg, k_coarse<R>, p.args));
 }
 
 template <typename R>
 static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& plan, int nu, long long big,
-                        int wfrom, double* rz, bool& need_dot) {
+                        int wfrom, double* rz) {
     cudaStream_t s = h->stream;
-    const dim3 sb(SX, SY);
+    const bool pdl = h->timing_mask == 0;
     if (l >= plan.l0) {
-        if (l == 0) need_dot = false;
-        launch_coarse(h, plan, l == 0 ? KC_SMOOTH0 : KC_BOTTOM, l == 0 ? rz : nullptr, s);
+        launch_coarse(h, plan, l == 0 ? KC_SMOOTH0 : KC_BOTTOM, l == 0 ? rz : nullptr, l > 0 && pdl, s);
         return;
     }
     Level<R>& L = H.lv[l];
@@ -1464,18 +1630,9 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& pl
     const int cls = l == 0 ? KC_SMOOTH0 : KC_MGREST;
     const bool is_big = ncells(g) >= big;
     const int gamma = (l >= wfrom && !is_big) ? 2 : 1;
-    dim3 hb, hg;
-    rbgs_grid<R>(g, hg, hb);
-    auto half_pre = [&](bool zero) {
-        if (zero)
-            WPF_LAUNCH(h, cls, k_rbgs_first<R><<<cell_grid(g.nx, g.ny, g.nz), cell_block(), 0, s>>>(g, L.idiag, L.x, L.b));
-        else
-            WPF_LAUNCH(h, cls, k_rbgs<R><<<hg, hb, 0, s>>>(g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, 0));
-        WPF_LAUNCH(h, cls, k_rbgs<R><<<hg, hb, 0, s>>>(g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, 1));
-    };
-    auto half_post = [&]() {
-        WPF_LAUNCH(h, cls, k_rbgs<R><<<hg, hb, 0, s>>>(g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, 1));
-        WPF_LAUNCH(h, cls, k_rbgs<R><<<hg, hb, 0, s>>>(g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, 0));
+    auto restrict_from = [&](const R* x) {
+        WPF_LAUNCH(h, KC_MGREST, launch_behind(pdl, k_resid_restrict<R>, cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), s,
+                                               g, C.g, L.cx, L.cy, L.cz, L.diag, L.idiag, x, L.b, C.b));
     };
     if (is_big) {
         R* buf[2] = {L.xs, L.x};
@@ -1484,34 +1641,45 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& pl
             R* out = buf[it & 1];
             launch_sweep(h, H, l, cls, it == 0, in, out, 0, nullptr);
         }
-        const R* pre_end = buf[(nu - 1) & 1];
-        WPF_LAUNCH(h, KC_MGREST, k_resid_restrict<R><<<cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), 0, s>>>(
-            g, C.g, L.cx, L.cy, L.cz, L.diag, pre_end, L.b, C.b));
-        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr, need_dot);
+        restrict_from(buf[(nu - 1) & 1]);
+        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr);
         for (int it = 0; it < nu; ++it) {
             const int w = nu + it;   // sweep number in the cycle: writes buf[w & 1]
             R* in = buf[(w + 1) & 1];
             R* out = buf[w & 1];
             const bool last0 = (l == 0 && it == nu - 1 && rz);
-            if (last0) need_dot = false;
             if (it == 0)   // the coarse correction, into the first post-sweep's input
                 launch_prolong<R>(h, g, C.g, L.idiag, in, C.x, s);
             launch_sweep(h, H, l, cls, false, in, out, 1, last0 ? rz : nullptr);
         }
         return;
     }
-    for (int it = 0; it < nu; ++it) half_pre(it == 0);
+    dim3 hb, hg;
+    rbgs_grid<R>(g, hg, hb);
+    auto half = [&](int color) {
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs<R>, hg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, color));
+    };
+    // (the first launch on level 0 is the cycle's first)
+    WPF_LAUNCH(h, cls, launch_behind(pdl && l > 0, k_rbgs_zero<R>, hg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b));
+    for (int it = 1; it < nu; ++it) { half(0); half(1); }
     for (int rep = 0; rep < gamma; ++rep) {
-        WPF_LAUNCH(h, KC_MGREST, k_resid_restrict<R><<<cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), 0, s>>>(
-            g, C.g, L.cx, L.cy, L.cz, L.diag, L.x, L.b, C.b));
-        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr, need_dot);
-        launch_prolong<R>(h, g, C.g, L.idiag, L.x, C.x, s);
-        if (rep + 1 < gamma) {
-            for (int it = 0; it < nu; ++it) half_post();
-            for (int it = 0; it < nu; ++it) half_pre(false);
+        restrict_from(L.x);
+        cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr);
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_corr<R>, hg, hb, s, g, C.g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, C.x));
+        for (int it = 1; it < nu; ++it) { half(0); half(1); }
+        if (rep + 1 < gamma) {   // the post-sweeps' last red half-sweep is the pre-sweeps' first
+            for (int it = 0; it < nu; ++it) { half(0); half(1); }
         }
     }
-    for (int it = 0; it < nu; ++it) half_post();
+    if (l == 0 && rz) {
+        const long long plane = (long long)hg.x * hg.y;
+        const long long nz = (long long)h->nsm * 8 / plane;
+        dim3 dg = hg;
+        dg.z = (unsigned)(nz < 1 ? 1 : (nz < hg.z ? nz : hg.z));
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_dot<R>, dg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, rz));
+        return;
+    }
+    half(0);
 }
 
 template <typename R>
@@ -1519,12 +1687,7 @@ static void vcycle(wpf_handle* h, Hierarchy<R>& H, int nu, double* rz) {
     const long long big = h->opts.sweep_min_cells > 0 ? h->opts.sweep_min_cells : BIG_CELLS;
     const int wfrom = h->opts.w_from_level > 0 ? h->opts.w_from_level : 2;
     CoarsePlan<R> plan = coarse_plan(h, H, nu, big, wfrom);
-    bool need_dot = rz != nullptr;
-    cycle_level(h, H, 0, plan, nu, big, wfrom, rz, need_dot);
-    if (need_dot) {
-        const Grid& g = H.lv[0].g;
-        WPF_LAUNCH(h, KC_VEC, k_dot<R><<<row_blocks(h, g), RB, 0, h->stream>>>(g, H.r, H.z, rz));
-    }
+    cycle_level(h, H, 0, plan, nu, big, wfrom, rz);
 }
 
 template <typename R>
