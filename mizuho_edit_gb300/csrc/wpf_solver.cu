@@ -1166,8 +1166,7 @@ __global__ void __launch_bounds__(RB) k_apply_p(Grid g, const R* __restrict__ cx
                                                 const double* __restrict__ rz_old, int first_a,
                                                 const int* it, double* acc,
                                                 const float* __restrict__ w = nullptr,
-                                                const double* __restrict__ gam = nullptr,
-                                                double* wq = nullptr) {
+                                                const double* __restrict__ gam = nullptr) {
     __shared__ R sbeta, sgam;
     __shared__ int sfirst, sodd, suse;
     if (threadIdx.x == 0) {
@@ -1191,7 +1190,7 @@ __global__ void __launch_bounds__(RB) k_apply_p(Grid g, const R* __restrict__ cx
     const R* __restrict__ pold = sodd ? pnew_a : pold_a;
     R* __restrict__ pnew = sodd ? pold_a : pnew_a;
     const long long sy = g.P, sz = g.S;
-    R d = 0, dw = 0;
+    R d = 0;
     ROW_LOOP(g) {
         const long long n = g.at(i, j, k);
         auto P = [&](long long m) {
@@ -1205,10 +1204,113 @@ __global__ void __launch_bounds__(RB) k_apply_p(Grid g, const R* __restrict__ cx
         pnew[n] = pc;
         q[n] = v;
         d += pc * v;
-        if (usew) dw += (R)w[n] * v;
     }
     block_add(d, acc);
-    if (usew && wq) block_add(dw, wq);
+}
+
+// The same for FP64.  A block forms p_new once on a 32 x 8 x AZ brick and the
+// cells around it (all loads in flight together), keeps it in shared memory and
+// takes the stencil from there: two multiply-adds a cell for p_new against the
+// seven of forming it at every neighbour.  The FP64 pipe bounds the kernel
+// (two multiply-adds a cycle and SM): 96x80x72 38.1 -> 17.1 us, 64^3 22.1 -> 10.5.  In FP32, where
+// it does not, bricks are the slower form: 100x90x110 10.4 -> 14.5 us, 256^3
+// 125 -> 146 us.  Blocks walk the bricks (few atomics on the sum's address).
+constexpr int AX = 32, AY = 8, AZ = 4;
+template <typename R>
+__global__ void __launch_bounds__(AX * AY) k_apply_p_brick(Grid g, const R* __restrict__ cx,
+                                                     const R* __restrict__ cy,
+                                                     const R* __restrict__ cz,
+                                                     const R* __restrict__ diag,
+                                                     const R* __restrict__ z,
+                                                     R* pold_a, R* pnew_a, R* __restrict__ q,
+                                                     const double* __restrict__ rz_new,
+                                                     const double* __restrict__ rz_old, int first_a,
+                                                     const int* it, double* acc,
+                                                     const float* __restrict__ w = nullptr,
+                                                     const double* __restrict__ gam = nullptr) {
+    constexpr int HX = AX + 2, HY = AY + 2, HZ = AZ + 2, NT = AX * AY;
+    constexpr int NP = (HX * HY * HZ + NT - 1) / NT;
+    __shared__ R p[HZ][HY][HX];
+    __shared__ R sbeta, sgam;
+    __shared__ int sfirst, sodd, suse;
+    if (threadIdx.x == 0) {
+        int f = first_a, odd = 0;
+        if (it) {
+            const int v = *it;
+            f = v == 0;
+            odd = v & 1;
+        }
+        sfirst = f;
+        sodd = odd;
+        sbeta = f ? (R)0 : (R)(*rz_new / *rz_old);
+        const double gv = (w && gam) ? *gam : __longlong_as_double(0x7ff8000000000000LL);
+        suse = gv == gv;   // the learned coarse space is on (k_cc_pre)
+        sgam = suse ? (R)gv : (R)0;
+    }
+    __syncthreads();
+    const R beta = sbeta;
+    const R gm = sgam;
+    const bool first = sfirst, usew = suse;
+    const R* __restrict__ pold = sodd ? pnew_a : pold_a;
+    R* __restrict__ pnew = sodd ? pold_a : pnew_a;
+    const long long sy = g.P, sz = g.S;
+    const int tx = threadIdx.x % AX, ty = threadIdx.x / AX;
+    const int bx = (g.nx + AX - 1) / AX, by = (g.ny + AY - 1) / AY, bz = (g.nz + AZ - 1) / AZ;
+    R d = 0;
+    for (int t = blockIdx.x; t < bx * by * bz; t += gridDim.x) {
+        const int i0 = (t % bx) * AX, j0 = (t / bx % by) * AY, k0 = t / (bx * by) * AZ;   // halo cell 0 of the brick
+        R v[NP], o[NP];
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int e = threadIdx.x + u * NT, r = e / HX;
+            const int i = i0 + e - r * HX, j = j0 + r % HY, k = k0 + r / HY;
+            v[u] = 0;
+            o[u] = 0;
+            if (e < HX * HY * HZ && i <= g.nx + 1 && j <= g.ny + 1 && k <= g.nz + 1) {
+                const long long m = g.at(i, j, k);
+                v[u] = z[m];
+                if (usew) v[u] += gm * (R)w[m];
+                if (!first) o[u] = pold[m];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int e = threadIdx.x + u * NT;
+            if (e < HX * HY * HZ) (&p[0][0][0])[e] = first ? v[u] : v[u] + beta * o[u];
+        }
+        __syncthreads();
+        const int i = i0 + 1 + tx, j = j0 + 1 + ty;
+        if (i <= g.nx && j <= g.ny) {
+#pragma unroll
+            for (int c = 0; c < AZ; ++c) {
+                const int k = k0 + 1 + c;
+                if (k > g.nz) break;
+                const long long n = g.at(i, j, k);
+                const R pc = p[c + 1][ty + 1][tx + 1];
+                const R qv = diag[n] * pc - (cx[n] * p[c + 1][ty + 1][tx + 2] + cx[n - 1] * p[c + 1][ty + 1][tx] +
+                                             cy[n] * p[c + 1][ty + 2][tx + 1] + cy[n - sy] * p[c + 1][ty][tx + 1] +
+                                             cz[n] * p[c + 2][ty + 1][tx + 1] + cz[n - sz] * p[c][ty + 1][tx + 1]);
+                pnew[n] = pc;
+                q[n] = qv;
+                d += pc * qv;
+            }
+        }
+        __syncthreads();
+    }
+    block_add(d, acc);
+}
+// k_apply_p in the form of the precision.
+template <typename R, typename... A>
+static void launch_apply(wpf_handle* h, const Grid& g, cudaStream_t s, A... a) {
+    if constexpr (sizeof(R) == 4) {
+        WPF_LAUNCH(h, KC_APPLY, k_apply_p<R><<<row_blocks_for(h, g, k_apply_p<R>), RB, 0, s>>>(g, a...));
+    } else {
+        const long long bricks = (long long)((g.nx + AX - 1) / AX) * ((g.ny + AY - 1) / AY) * ((g.nz + AZ - 1) / AZ);
+        const int per_sm = h->opts.row_blocks_per_sm > 0 ? h->opts.row_blocks_per_sm
+                                                         : resident_blocks((const void*)k_apply_p_brick<R>, AX * AY, 0, 8);
+        const long long cap = (long long)h->nsm * per_sm;
+        WPF_LAUNCH(h, KC_APPLY, k_apply_p_brick<R><<<(unsigned)(bricks < cap ? bricks : cap), AX * AY, 0, s>>>(g, a...));
+    }
 }
 
 // alpha = rz/pq; x += alpha p (x = alpha p when first, unless x_set); r -= alpha q; accumulate r.r
@@ -1812,9 +1914,8 @@ static int pcg(wpf_handle* h, Hierarchy<R>& H, double tol, int maxit, int nu, in
             WPF_LAUNCH(h, KC_OTHER, k_cc_mu<<<1, 32, 0, s>>>(nullptr, d));
         }
         WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 2 * sizeof(double), s));   // S_PQ, S_RR
-        WPF_LAUNCH(h, KC_APPLY, k_apply_p<R><<<row_blocks_for(h, g, k_apply_p<R>), RB, 0, s>>>(g, L0.cx, L0.cy, L0.cz, L0.diag, H.z, pold, pnew,
-                                                 H.q, d + S_RZ0 + cur, d + S_RZ0 + (cur ^ 1),
-                                                 it == 0, nullptr, d + S_PQ, wc, d + S_GAM));
+        launch_apply<R>(h, g, s, L0.cx, L0.cy, L0.cz, L0.diag, H.z, pold, pnew, H.q, d + S_RZ0 + cur, d + S_RZ0 + (cur ^ 1),
+                        (int)(it == 0), (const int*)nullptr, d + S_PQ, wc, d + S_GAM);
         WPF_LAUNCH(h, KC_VEC, k_update_xr<R><<<rb, RB, 0, s>>>(g, H.x, H.r, pnew, pnew, H.q, d + S_RZ0 + cur,
                                                    d + S_PQ, it == 0, nullptr, d + S_RR, wc != nullptr));
         rc = read_slot(h, S_PQ, 2);
@@ -2459,9 +2560,8 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
         WPF_LAUNCH(h, KC_OTHER, k_cc_mu<<<1, 32, 0, s>>>(c, d));
     }
     WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 2 * sizeof(double), s));   // PQ, RR
-    WPF_LAUNCH(h, KC_APPLY, k_apply_p<R><<<row_blocks_for(h, g, k_apply_p<R>), RB, 0, s>>>(g, L0.cx, L0.cy, L0.cz, L0.diag, H.z, H.p2, H.p, H.q,
-                                                             d + S_RZ1, d + S_RZ0, 0, &c->it, d + S_PQ, wc,
-                                                             d + S_GAM));
+    launch_apply<R>(h, g, s, L0.cx, L0.cy, L0.cz, L0.diag, H.z, H.p2, H.p, H.q,
+                    d + S_RZ1, d + S_RZ0, 0, &c->it, d + S_PQ, wc, d + S_GAM);
     WPF_LAUNCH(h, KC_VEC, k_update_xr<R><<<rb, RB, 0, s>>>(g, H.x, H.r, H.p, H.p2, H.q, d + S_RZ1, d + S_PQ, 0,
                                                            &c->it, d + S_RR, wc != nullptr));
     WPF_LAUNCH(h, KC_OTHER, k_ctl_pcg_check<<<1, 32, 0, s>>>(c, d, h->opts.max_inner, h_it));
