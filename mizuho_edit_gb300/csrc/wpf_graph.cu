@@ -150,8 +150,9 @@ int gb_add_split(wpf_handle* h, GraphBuilder& b, bool* added) {
 // The dt law of wPFAW3D.f90:2227-2230, dt = dt_c * min(dt_a, taumin), with
 // dt_c = tfac * dx^2 / (2 eps^2) and dt_a = eps^2 / D, taumin from the key the
 // previous update left in S_TAUMIN_KEY; the extrapolation coefficients of
-// ws_coeffs for two held increments; the solve's control state and slots reset.
-__global__ void k_step_begin(StepCtl* c, double* dsc, double dt_c, double dt_a) {
+// ws_coeffs for two held increments; whether the least-squares start is taken;
+// the solve's control state and slots reset.
+__global__ void k_step_begin(StepCtl* c, double* dsc, double dt_c, double dt_a, double rtol, long long cells) {
     if (threadIdx.x) return;
     const double tm = dkey_inv(reinterpret_cast<const unsigned long long*>(dsc)[S_TAUMIN_KEY]);
     const double dt = dt_c * (dt_a < tm ? dt_a : tm);
@@ -165,7 +166,11 @@ __global__ void k_step_begin(StepCtl* c, double* dsc, double dt_c, double dt_a) 
         c->wa = (float)(hn / h1 + q / h1);
         c->wb = (float)(-q / h2);
     }
-    c->bnorm_prev = c->bnorm;   // the least-squares start's scale (k_ctl_ls_begin)
+    c->bnorm_prev = c->bnorm;   // the least-squares start's scale
+    c->ls = ws_ls_wanted(c->rp_rel, c->bnorm_prev, rtol) ? 1 : 0;
+    c->ls_skip = 0;
+    dsc[S_LSSCALE] = ws_ls_scale(c->bnorm_prev, rtol, cells);
+    for (int q = S_LS0; q <= S_LS5; ++q) dsc[q] = 0.0;
     c->bnorm = c->relres = c->relres0 = c->r0 = c->tol = 0.0;
     c->pass = c->outer = c->inner = c->it = c->need_pcg = c->accept = c->used = c->pcgs = c->net_runs = 0;
     c->alpha = 0.f;
@@ -236,7 +241,8 @@ int step_graph_capture(wpf_handle* h, GraphBuilder& b, StepCounts* n) {
     int rc;
     if ((rc = gb_begin(b))) return rc;
     long long l0 = h->nlaunch;
-    WPF_LAUNCH(h, KC_OTHER, k_step_begin<<<1, 32, 0, s>>>(c, h->dsc, dt_c, dt_a));
+    WPF_LAUNCH(h, KC_OTHER, k_step_begin<<<1, 32, 0, s>>>(c, h->dsc, dt_c, dt_a, h->opts.rtol,
+                                                          (long long)h->g.nx * h->g.ny * h->g.nz));
     // the extrapolated start needs only the dt law's coefficients: it is
     // built beside calcPermeability (HBM-bound beside FP64-bound)
     if ((rc = ws_capture_early(h, &h->ws_early))) return rc;

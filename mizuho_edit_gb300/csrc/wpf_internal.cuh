@@ -136,7 +136,28 @@ struct StepCtl {
     int ls_skip;             // its predicted residual meets rtol: pass 0's residual kernel is skipped
     double rp_rel;           // ||r(p)|| / ||b|| of the last pass 0 (kept across steps)
     double bnorm_prev;       // ||b|| of the last step (the least-squares dots' scale)
+    unsigned ticket;         // blocks of the running kernel that are done (last_block)
 };
+
+// Whether the least-squares start is taken this step: when the previous
+// pressure's residual under the new T (the last pass 0's record) is below
+// LS_WINDOW rtol.  Measured at 256^3 (time-steps/s, least-squares start
+// always / below 100 rtol / below 10 rtol): kwh 10^3 early in the run, p at
+// ~46 rtol, 329.5 / 329.4 / 292.1; late, p at ~1.7 rtol, 363.5 / 362.9 /
+// 355.2; kwh 20 early, p at ~390 rtol, 314.7 / 339.8 / 339.5 (the fit
+// costs its pass and saves no iteration there); kwh 20 late, p at ~30 rtol,
+// 336.6 / 336.6 / 264.4.  And the power of two that brings values of the
+// size rtol ||b|| / sqrt(cells) to ~1.
+constexpr double LS_WINDOW = 100.0;
+__host__ __device__ inline bool ws_ls_wanted(double rp_rel, double bnorm_prev, double rtol) {
+    return rp_rel > 0.0 && rp_rel < LS_WINDOW * rtol && bnorm_prev > 0.0;
+}
+__host__ __device__ inline double ws_ls_scale(double bnorm_prev, double rtol, long long cells) {
+    const double v = bnorm_prev * rtol / sqrt((double)(cells > 0 ? cells : 1));
+    int e = (v > 0.0 && v == v) ? ilogb(v) : 0;
+    e = e < -100 ? -100 : (e > 100 ? 100 : e);
+    return ldexp(1.0, -e);
+}
 
 // Builds a CUDA graph from stream-captured segments and conditional nodes.
 // `graph` is the graph being extended (the top graph or a conditional body),

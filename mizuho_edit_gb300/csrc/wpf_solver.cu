@@ -55,6 +55,119 @@ constexpr int SX = 32, SY = 8;   // sweep tile (x, y); the z chunk is chosen per
 constexpr int FX = SX + 4, FY = SY + 4;    // shared footprint: tile + 2-cell ring
 
 // ---------------------------------------------------------------------------
+// Control of the device-resident step.  The decisions between kernels (whether
+// a start is accepted, a pass or an iteration follows) are taken by the last
+// block of the kernel whose sums they need: a kernel of one thread for each
+// cost a launch, 1.2-1.7 us, about 17 of them a step.  The sums were added by
+// atomics while the block's own L1 may hold their line from before, so they
+// are read through L2.
+// ---------------------------------------------------------------------------
+// Thread 0 of every block, after its last atomic and its last read of *c: the
+// ticket releases this thread's atomics and the last one acquires them all.
+__device__ __forceinline__ bool last_block(StepCtl* c) {
+    unsigned t;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(&c->ticket) : "memory");
+    if (t != gridDim.x * gridDim.y * gridDim.z - 1) return false;
+    c->ticket = 0;
+    return true;
+}
+
+// After a refinement pass's residual (S_RR64, S_BB64): the pass logic of solve_impl.
+struct PassCtl {
+    StepCtl* c = nullptr;   // null: none (the host takes the decision)
+    double rtol = 0.0, inner_rtol = 0.0;
+    int max_outer = 0, mixed = 0;
+    cudaGraphConditionalHandle h = 0;
+};
+__device__ __noinline__ void ctl_pass(const PassCtl& a, const double* dsc) {
+    StepCtl* c = a.c;
+    const double rr = __ldcg(dsc + S_RR64), bb = __ldcg(dsc + S_BB64);
+    const int pass = c->pass;
+    int cont = 0, pcg = 0;
+    if (c->status != WPF_ERR_NONFINITE) {   // else a PCG of the last pass broke down
+        // ||b|| from pass 0, and from the verification pass after a pass 0
+        // whose residual the least-squares prediction replaced (the exact one)
+        if (pass == 0 || bb > 0.0) c->bnorm = sqrt(bb);
+        const double bnorm = c->bnorm;
+        const double rnorm = sqrt(rr);
+        const double relres = bnorm > 0.0 ? rnorm / bnorm : rnorm;
+        c->relres = relres;
+        if (pass == 0) c->relres0 = relres;
+        if (!(relres == relres) || isinf(relres)) {
+            c->status = WPF_ERR_NONFINITE;
+        } else if (relres <= a.rtol) {
+            // an accepted start that already meets rtol: add it, verify by a plain pass
+            if (c->accept && pass < a.max_outer) cont = 1;
+            else c->status = WPF_OK;
+        } else if (pass < a.max_outer) {
+            c->outer = pass + 1;
+            const double want = 0.5 * a.rtol / relres;
+            c->tol = a.mixed ? fmax(a.inner_rtol, want) : want;
+            cont = 1;
+            pcg = 1;
+        }
+    }
+    c->need_pcg = pcg;
+    cudaGraphSetConditional(a.h, cont);
+}
+
+// PCG prologue (r.r in S_RR) and the test after an iteration.
+struct PcgCtl {
+    StepCtl* c = nullptr;
+    double* dsc = nullptr;
+    int maxit = 0;
+    cudaGraphConditionalHandle h = 0;
+};
+// The iterations run when the pass needs a PCG and ||r_0|| > 0 (pcg's early return).
+__device__ __noinline__ void ctl_pcg_start(const PcgCtl& a) {
+    StepCtl* c = a.c;
+    int run = 0;
+    c->it = 0;
+    if (c->need_pcg) {
+        ++c->pcgs;
+        const double r0 = sqrt(__ldcg(a.dsc + S_RR));
+        c->r0 = r0;
+        if (r0 > 0.0) run = 1;
+        else if (r0 != 0.0) c->status = WPF_ERR_NONFINITE;
+    }
+    a.dsc[S_RR] = 0.0;
+    cudaGraphSetConditional(a.h, run);
+}
+// pcg's convergence test; this r.z becomes the previous, the iteration's sums are cleared.
+__device__ __noinline__ void ctl_pcg_check(const PcgCtl& a) {
+    StepCtl* c = a.c;
+    const double rr = __ldcg(a.dsc + S_RR), rz = __ldcg(a.dsc + S_RZ1), tol = c->tol, r0 = c->r0;   // (all in flight)
+    const int it = c->it + 1, inner = c->inner + 1;
+    const double rn = sqrt(rr);
+    const bool bad = !(rn == rn) || isinf(rn);
+    const int cont = !bad && !(rn <= tol * r0) && it < a.maxit;
+    if (bad) c->status = WPF_ERR_NONFINITE;
+    c->it = it;
+    c->inner = inner;
+    a.dsc[S_RZ0] = rz;
+    a.dsc[S_RZ1] = a.dsc[S_PQ] = a.dsc[S_RR] = 0.0;
+    cudaGraphSetConditional(a.h, cont);
+}
+// Between passes: the start is consumed, the next pass's residual slots cleared.
+__device__ __noinline__ void ctl_advance(StepCtl* c, double* dsc) {
+    c->accept = 0;
+    ++c->pass;
+    for (int q = 0; q < 5; ++q) dsc[S_RR64 + q] = 0.0;
+}
+__device__ __noinline__ void ctl_accept(StepCtl* c, double* dsc) {
+    const double rstart = __ldcg(dsc + S_RR64), r0 = __ldcg(dsc + S_RR0WS), bb = __ldcg(dsc + S_BB64);
+    if (bb > 0.0) c->rp_rel = sqrt(r0 / bb);   // for the next step's least-squares start
+    if (rstart <= r0 && rstart == rstart) {
+        c->accept = 1;
+        c->used = 1;
+    } else {
+        c->accept = 0;
+        c->used = -1;
+        for (int q = 0; q < 5; ++q) dsc[S_RR64 + q] = 0.0;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // FP64 outer residual.  r = qterm + sum_f T_f (p_nb - p_c) on free cells, 0 on
 // Dirichlet cells; accumulates ||r||^2 and, when want_b, ||b_ref||^2 with
 // b_ref the reference right-hand side (:803-825, :852-931).
@@ -96,13 +209,17 @@ __global__ void __launch_bounds__(RB) k_resid64(Grid g, const double* __restrict
                                                 const int* skip = nullptr,
                                                 float* __restrict__ zero_out = nullptr,
                                                 double* __restrict__ rk_out = nullptr,
-                                                const int* want_b_dev = nullptr) {
+                                                const int* want_b_dev = nullptr, PassCtl pc = {}) {
     // skip: a device flag that, when set, makes the launch a no-op (the
     // device-resident step launches this pass unconditionally); zero_out: a
     // field whose interior is cleared on the way; rk_out: the residual kept
     // in FP64 for the next solve's pass 0; want_b_dev: a device flag that
-    // also asks for ||b|| (set when pass 0's residual was a prediction)
-    if (skip && *skip) return;
+    // also asks for ||b|| (set when pass 0's residual was a prediction); pc:
+    // the pass's convergence test, by the last block (which changes neither flag)
+    if (skip && *skip) {
+        if (pc.c && blockIdx.x == 0 && threadIdx.x == 0) ctl_pass(pc, dsc);
+        return;
+    }
     if (want_b_dev && *want_b_dev) want_b = 1;
     double rr = 0.0, bb = 0.0;
     R rrr = 0;
@@ -145,6 +262,7 @@ __global__ void __launch_bounds__(RB) k_resid64(Grid g, const double* __restrict
     rr += (double)rrr;
     block_add(rr, dsc + S_RR64);
     if (want_b) block_add(bb, dsc + S_BB64);
+    if (pc.c && threadIdx.x == 0 && last_block(pc.c)) ctl_pass(pc, dsc);
 }
 
 // p += e on the interior (e is zero on dead cells).
@@ -199,6 +317,43 @@ __device__ __forceinline__ R apply_l0(const R* __restrict__ cx, const R* __restr
             cz[n - sz] * from_f32<R>(e[n - sz]));
 }
 
+// The 2x2 normal equations of the least-squares start; a one-direction fit
+// when d2 adds nothing to d1, and the given (a, b) kept when neither fits.
+__host__ __device__ inline void ws_ls_solve(const double* m, float* a, float* b) {
+    const double ra = m[0], rb = m[1], aa = m[2], ab = m[3], bb = m[4];
+    const double det = aa * bb - ab * ab;
+    if (aa > 0.0 && bb > 0.0 && det > 1e-6 * aa * bb && det == det && ra == ra && rb == rb) {
+        *a = (float)((ra * bb - rb * ab) / det);
+        *b = (float)((aa * rb - ab * ra) / det);
+    } else if (aa > 0.0 && ra == ra) {
+        *a = (float)(ra / aa);
+        *b = 0.f;
+    }
+}
+// ||r(p) - A'(a d1 + b d2)||^2 from the dots (scaled like them)
+__host__ __device__ inline double ws_ls_predict(const double* m, double a, double b) {
+    return m[5] - 2.0 * (a * m[0] + b * m[1]) + a * a * m[2] + 2.0 * a * b * m[3] + b * b * m[4];
+}
+// The predicted start residual at or below LS_SKIP rtol ||b|| (with the last
+// step's ||b||) skips pass 0's residual kernel: the start is accepted on the
+// prediction and the plain FP64 verification pass decides as always.
+constexpr double LS_SKIP = 0.8;
+
+// (rtol < 0: never skip)
+__device__ __noinline__ void ctl_ws_ls(StepCtl* c, double* dsc, double rtol) {
+    double m[6];
+    for (int q = 0; q < 6; ++q) m[q] = __ldcg(dsc + S_LS0 + q);
+    ws_ls_solve(m, &c->wa, &c->wb);
+    const double s = dsc[S_LSSCALE], bn = c->bnorm_prev;
+    const double pred = fmax(ws_ls_predict(m, c->wa, c->wb), 0.0) / (s * s);
+    if (sqrt(pred) <= LS_SKIP * rtol * bn) {   // the norms pass 0 would have given
+        c->ls_skip = 1;
+        dsc[S_RR64] = pred;
+        dsc[S_RR0WS] = m[5] / (s * s);
+        dsc[S_BB64] = bn * bn;
+    }
+}
+
 // The least-squares start (the default; WPF_SOLVER_FIXED_START keeps the
 // fixed coefficients): the five dots of min_{a,b} ||r - A'(a d1 + b d2)||, r
 // the kept FP64 residual of p under this step's transmissibilities, A' the
@@ -206,13 +361,14 @@ __device__ __forceinline__ R apply_l0(const R* __restrict__ cx, const R* __restr
 // scaled by a power of two s (from the last step's ||b||, so that they are
 // O(1) at the tolerance's scale) and the dots accumulated in FP32 per thread,
 // FP64 across threads; the solution does not depend on s.  Dirichlet cells
-// carry no residual.  c non-null (the step graph): a no-op unless c->ls.
+// carry no residual.  c non-null (the step graph): a no-op unless c->ls; the
+// last block solves for the coefficients.
 template <typename R>
 __global__ void __launch_bounds__(RB) k_ws_ls_dots(Grid g, const R* __restrict__ cx, const R* __restrict__ cy,
                                                    const R* __restrict__ cz, const R* __restrict__ diag,
                                                    const uint8_t* __restrict__ fl, const float* __restrict__ d1,
                                                    const float* __restrict__ d2, const double* __restrict__ rk,
-                                                   const StepCtl* c, double scale, double* dsc) {
+                                                   StepCtl* c, double scale, double rtol, double* dsc) {
     if (c && !c->ls) return;
     const double s = c ? dsc[S_LSSCALE] : scale;
     const float sf = (float)s;
@@ -237,67 +393,7 @@ __global__ void __launch_bounds__(RB) k_ws_ls_dots(Grid g, const R* __restrict__
     block_add((double)ab, dsc + S_LS0 + 3);
     block_add((double)bb, dsc + S_LS0 + 4);
     block_add((double)rr, dsc + S_LS0 + 5);
-}
-
-// The 2x2 normal equations of the least-squares start; a one-direction fit
-// when d2 adds nothing to d1, and the given (a, b) kept when neither fits.
-__host__ __device__ inline void ws_ls_solve(const double* m, float* a, float* b) {
-    const double ra = m[0], rb = m[1], aa = m[2], ab = m[3], bb = m[4];
-    const double det = aa * bb - ab * ab;
-    if (aa > 0.0 && bb > 0.0 && det > 1e-6 * aa * bb && det == det && ra == ra && rb == rb) {
-        *a = (float)((ra * bb - rb * ab) / det);
-        *b = (float)((aa * rb - ab * ra) / det);
-    } else if (aa > 0.0 && ra == ra) {
-        *a = (float)(ra / aa);
-        *b = 0.f;
-    }
-}
-// ||r(p) - A'(a d1 + b d2)||^2 from the dots (scaled like them)
-__host__ __device__ inline double ws_ls_predict(const double* m, double a, double b) {
-    return m[5] - 2.0 * (a * m[0] + b * m[1]) + a * a * m[2] + 2.0 * a * b * m[3] + b * b * m[4];
-}
-// The predicted start residual at or below LS_SKIP rtol ||b|| (with the last
-// step's ||b||) skips pass 0's residual kernel: the start is accepted on the
-// prediction and the plain FP64 verification pass decides as always.
-constexpr double LS_SKIP = 0.8;
-
-// Whether the least-squares start is taken this step: when the previous
-// pressure's residual under the new T (the last pass 0's record) is below
-// LS_WINDOW rtol.  Measured at 256^3 (time-steps/s, least-squares start
-// always / below 100 rtol / below 10 rtol): kwh 10^3 early in the run, p at
-// ~46 rtol, 329.5 / 329.4 / 292.1; late, p at ~1.7 rtol, 363.5 / 362.9 /
-// 355.2; kwh 20 early, p at ~390 rtol, 314.7 / 339.8 / 339.5 (the fit
-// costs its pass and saves no iteration there); kwh 20 late, p at ~30 rtol,
-// 336.6 / 336.6 / 264.4.  And the power of two that brings values of the
-// size rtol ||b|| / sqrt(cells) to ~1.
-constexpr double LS_WINDOW = 100.0;
-__host__ __device__ inline bool ws_ls_wanted(double rp_rel, double bnorm_prev, double rtol) {
-    return rp_rel > 0.0 && rp_rel < LS_WINDOW * rtol && bnorm_prev > 0.0;
-}
-__host__ __device__ inline double ws_ls_scale(double bnorm_prev, double rtol, long long cells) {
-    const double v = bnorm_prev * rtol / sqrt((double)(cells > 0 ? cells : 1));
-    int e = (v > 0.0 && v == v) ? ilogb(v) : 0;
-    e = e < -100 ? -100 : (e > 100 ? 100 : e);
-    return ldexp(1.0, -e);
-}
-__global__ void k_ctl_ls_begin(StepCtl* c, double* dsc, double rtol, long long cells) {
-    if (threadIdx.x) return;
-    c->ls = ws_ls_wanted(c->rp_rel, c->bnorm_prev, rtol) ? 1 : 0;
-    c->ls_skip = 0;
-    dsc[S_LSSCALE] = ws_ls_scale(c->bnorm_prev, rtol, cells);
-}
-// (rtol < 0: never skip)
-__global__ void k_ctl_ws_ls(StepCtl* c, double* dsc, double rtol) {
-    if (threadIdx.x || !c->ls) return;
-    ws_ls_solve(dsc + S_LS0, &c->wa, &c->wb);
-    const double s = dsc[S_LSSCALE], bn = c->bnorm_prev;
-    const double pred = fmax(ws_ls_predict(dsc + S_LS0, c->wa, c->wb), 0.0) / (s * s);
-    if (sqrt(pred) <= LS_SKIP * rtol * bn) {   // the norms pass 0 would have given
-        c->ls_skip = 1;
-        dsc[S_RR64] = pred;
-        dsc[S_RR0WS] = dsc[S_LS5] / (s * s);
-        dsc[S_BB64] = bn * bn;
-    }
+    if (c && threadIdx.x == 0 && last_block(c)) ctl_ws_ls(c, dsc, rtol);
 }
 
 // Pass-0 residual of the start p + e_ext: r0 = r(p) in FP64 exactly as
@@ -325,8 +421,12 @@ __global__ void __launch_bounds__(RB) k_resid64_ws(Grid g, const double* __restr
                                                    const float* __restrict__ e1,
                                                    R* __restrict__ rout, float* __restrict__ dnew,
                                                    double* dsc, const double* __restrict__ rk_in = nullptr,
-                                                   const int* skip = nullptr) {
-    if (skip && *skip) return;   // the least-squares start's prediction stands in (k_ctl_ws_ls)
+                                                   const int* skip = nullptr, StepCtl* c = nullptr) {
+    // c: the last block decides on the start (ctl_accept)
+    if (skip && *skip) {   // the least-squares start's prediction stands in (ctl_ws_ls)
+        if (c && blockIdx.x == 0 && threadIdx.x == 0) ctl_accept(c, dsc);
+        return;
+    }
     double rr1 = 0.0, rr0 = 0.0, bb = 0.0;
     R rr1r = 0;   // the same sum in R (with D)
     float rr0f = 0.f;               // ||r(p)||^2 in FP32 on the kept path (only the fallback test reads it)
@@ -398,6 +498,7 @@ __global__ void __launch_bounds__(RB) k_resid64_ws(Grid g, const double* __restr
     block_add(rr1, dsc + S_RR64);
     block_add(rr0, dsc + S_RR0WS);
     block_add(bb, dsc + S_BB64);
+    if (c && threadIdx.x == 0 && last_block(c)) ctl_accept(c, dsc);
 }
 
 // Accept the learned correction with step alpha: r -= alpha A'e_net,
@@ -1321,7 +1422,7 @@ __global__ void __launch_bounds__(RB) k_update_xr(Grid g, R* __restrict__ x, R* 
                                                   const R* __restrict__ q,
                                                   const double* __restrict__ rz,
                                                   const double* __restrict__ pq, int first_a,
-                                                  const int* it, double* acc, int x_set = 0) {
+                                                  const int* it, double* acc, int x_set = 0, PcgCtl pc = {}) {
     __shared__ R salpha;
     __shared__ int sfirst, sodd;
     if (threadIdx.x == 0) {
@@ -1342,17 +1443,19 @@ __global__ void __launch_bounds__(RB) k_update_xr(Grid g, R* __restrict__ x, R* 
         d += rn * rn;
     }
     block_add(d, acc);
+    if (pc.c && threadIdx.x == 0 && last_block(pc.c)) ctl_pcg_check(pc);
 }
 
 template <typename R>
 __global__ void __launch_bounds__(RB) k_dot(Grid g, const R* __restrict__ a,
-                                            const R* __restrict__ b, double* acc) {
+                                            const R* __restrict__ b, double* acc, PcgCtl pc = {}) {
     R d = 0;
     ROW_LOOP_U4(g) {
         const long long n = g.at(i, j, k);
         d += a[n] * b[n];
     }
     block_add(d, acc);
+    if (pc.c && threadIdx.x == 0 && last_block(pc.c)) ctl_pcg_start(pc);
 }
 
 // ---- the learned coarse space (WPF_SOLVER_NET_COARSE) ----------------------
@@ -2087,7 +2190,7 @@ static int solve_impl(wpf_handle* h, Hierarchy<R>& H, wpf_step_stats* st) {
                 WPF_CUDA(cudaMemsetAsync(h->dsc + S_LS0, 0, 6 * sizeof(double), s));
                 WPF_LAUNCH(h, KC_RESID64, k_ws_ls_dots<R><<<row_blocks_for(h, g, k_ws_ls_dots<R>), RB, 0, s>>>(
                     g, H.lv[0].cx, H.lv[0].cy, H.lv[0].cz, H.lv[0].diag, h->flags, h->ws[0],
-                    h->ws_hist >= 2 ? h->ws[1] : h->ws[0], rk_in, nullptr, sc, h->dsc));
+                    h->ws_hist >= 2 ? h->ws[1] : h->ws[0], rk_in, nullptr, sc, 0.0, h->dsc));
                 WPF_CUDA(cudaGetLastError());
                 if ((rc = read_slot(h, S_LS0, 6))) return rc;
                 ws_ls_solve(h->hsc + S_LS0, &wa, &wb);
@@ -2107,7 +2210,7 @@ static int solve_impl(wpf_handle* h, Hierarchy<R>& H, wpf_step_stats* st) {
                 auto* kern = rk_in ? k_resid64_ws<R, true> : k_resid64_ws<R, false>;
                 WPF_LAUNCH(h, KC_RESID64, kern<<<row_blocks_for(h, g, kern), RB, 0, s>>>(
                     g, h->pressure, h->T[0], h->T[1], h->T[2], h->flags, h->qterm, resid_dsum(h), H.lv[0].cx,
-                    H.lv[0].cy, H.lv[0].cz, H.lv[0].diag, h->ws_e[0], H.r, dnew, h->dsc, rk_in, nullptr));
+                    H.lv[0].cy, H.lv[0].cz, H.lv[0].diag, h->ws_e[0], H.r, dnew, h->dsc, rk_in, nullptr, nullptr));
                 WPF_CUDA(cudaGetLastError());
                 rc = read_slot(h, S_RR64, 5);
                 if (rc) return rc;
@@ -2261,20 +2364,6 @@ static int solve_impl(wpf_handle* h, Hierarchy<R>& H, wpf_step_stats* st) {
 
 // Extrapolated start: kept when its residual is below that of p (solve_impl's
 // fallback rule); else the slots are cleared for the plain pass-0 residual.
-__global__ void k_ctl_accept(StepCtl* c, double* dsc) {
-    if (threadIdx.x) return;
-    const double rstart = dsc[S_RR64], r0 = dsc[S_RR0WS];
-    if (dsc[S_BB64] > 0.0) c->rp_rel = sqrt(r0 / dsc[S_BB64]);   // for the next step's least-squares start
-    if (rstart <= r0 && rstart == rstart) {
-        c->accept = 1;
-        c->used = 1;
-    } else {
-        c->accept = 0;
-        c->used = -1;
-        for (int q = 0; q < 5; ++q) dsc[S_RR64 + q] = 0.0;
-    }
-}
-
 // Whether the learned correction is evaluated this step (net_gate on the
 // extrapolated start's residual): the condition of the net's IF node.
 __global__ void k_ctl_net_gate(StepCtl* c, const double* dsc, double rtol, int always,
@@ -2332,76 +2421,6 @@ __global__ void __launch_bounds__(RB) k_ws_take_net_dev(Grid g, const R* __restr
     }
 }
 
-// After a refinement pass's residual: the pass logic of solve_impl.
-__global__ void k_ctl_pass(StepCtl* c, const double* dsc, double rtol, double inner_rtol, int max_outer,
-                           int mixed, cudaGraphConditionalHandle h_pass) {
-    if (threadIdx.x) return;
-    const int pass = c->pass;
-    int cont = 0, pcg = 0;
-    if (c->status != WPF_ERR_NONFINITE) {   // else a PCG of the last pass broke down
-        // ||b|| from pass 0, and from the verification pass after a pass 0
-        // whose residual the least-squares prediction replaced (the exact one)
-        if (pass == 0 || dsc[S_BB64] > 0.0) c->bnorm = sqrt(dsc[S_BB64]);
-        const double bnorm = c->bnorm;
-        const double rnorm = sqrt(dsc[S_RR64]);
-        const double relres = bnorm > 0.0 ? rnorm / bnorm : rnorm;
-        c->relres = relres;
-        if (pass == 0) c->relres0 = relres;
-        if (!(relres == relres) || isinf(relres)) {
-            c->status = WPF_ERR_NONFINITE;
-        } else if (relres <= rtol) {
-            // an accepted start that already meets rtol: add it, verify by a plain pass
-            if (c->accept && pass < max_outer) cont = 1;
-            else c->status = WPF_OK;
-        } else if (pass < max_outer) {
-            c->outer = pass + 1;
-            const double want = 0.5 * rtol / relres;
-            c->tol = mixed ? fmax(inner_rtol, want) : want;
-            cont = 1;
-            pcg = 1;
-        }
-    }
-    c->need_pcg = pcg;
-    cudaGraphSetConditional(h_pass, cont);
-}
-
-// PCG prologue (r.r in S_RR): the iterations run when the pass needs a PCG
-// and ||r_0|| > 0 (pcg's early return).
-__global__ void k_ctl_pcg_start(StepCtl* c, const double* dsc, cudaGraphConditionalHandle h_it) {
-    if (threadIdx.x) return;
-    int run = 0;
-    c->it = 0;
-    if (c->need_pcg) {
-        ++c->pcgs;
-        const double r0 = sqrt(dsc[S_RR]);
-        c->r0 = r0;
-        if (r0 > 0.0) run = 1;
-        else if (r0 != 0.0) c->status = WPF_ERR_NONFINITE;
-    }
-    cudaGraphSetConditional(h_it, run);
-}
-
-// After a PCG iteration: pcg's convergence test; this r.z becomes the previous.
-__global__ void k_ctl_pcg_check(StepCtl* c, double* dsc, int maxit, cudaGraphConditionalHandle h_it) {
-    if (threadIdx.x) return;
-    const int it = ++c->it;
-    ++c->inner;
-    const double rn = sqrt(dsc[S_RR]);
-    int cont = 0;
-    if (!(rn == rn) || isinf(rn)) c->status = WPF_ERR_NONFINITE;
-    else if (!(rn <= c->tol * c->r0) && it < maxit) cont = 1;
-    dsc[S_RZ0] = dsc[S_RZ1];
-    cudaGraphSetConditional(h_it, cont);
-}
-
-// Between passes: the start is consumed, the next pass's residual slots cleared.
-__global__ void k_ctl_advance(StepCtl* c, double* dsc) {
-    if (threadIdx.x) return;
-    c->accept = 0;
-    ++c->pass;
-    for (int q = 0; q < 5; ++q) dsc[S_RR64 + q] = 0.0;
-}
-
 // p += x (when this pass ran PCG iterations) + e1 [+ alpha e2] (when the
 // accepted start is pending; e2 the learned correction, taken when alpha > 0);
 // dnew accumulates x.  The arithmetic of k_add_correction(_ws).
@@ -2410,7 +2429,7 @@ __global__ void __launch_bounds__(RB) k_add_correction_dev(Grid g, double* __res
                                                            const R* __restrict__ x,
                                                            const float* __restrict__ e1,
                                                            const float* __restrict__ e2,
-                                                           float* __restrict__ dnew, const StepCtl* c) {
+                                                           float* __restrict__ dnew, StepCtl* c, double* dsc) {
     __shared__ int suse;
     __shared__ float salpha;
     if (threadIdx.x == 0) {
@@ -2421,14 +2440,16 @@ __global__ void __launch_bounds__(RB) k_add_correction_dev(Grid g, double* __res
     __syncthreads();
     const int use = suse;
     const float alpha = salpha;
-    if (!use) return;
-    ROW_LOOP_U4(g) {
-        const long long n = g.at(i, j, k);
-        double inc = (use & 1) ? to_f64<R>(x[n]) : 0.0;
-        if (use & 2) inc += f32_to_f64(alpha > 0.f ? e1[n] + alpha * e2[n] : e1[n]);
-        pr[n] += inc;
-        if ((use & 1) && dnew) dnew[n] += to_f32<R>(x[n]);
+    if (use) {
+        ROW_LOOP_U4(g) {
+            const long long n = g.at(i, j, k);
+            double inc = (use & 1) ? to_f64<R>(x[n]) : 0.0;
+            if (use & 2) inc += f32_to_f64(alpha > 0.f ? e1[n] + alpha * e2[n] : e1[n]);
+            pr[n] += inc;
+            if ((use & 1) && dnew) dnew[n] += to_f32<R>(x[n]);
+        }
     }
+    if (threadIdx.x == 0 && last_block(c)) ctl_advance(c, dsc);
 }
 
 template <typename R>
@@ -2454,6 +2475,8 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
     int rc;
     if ((rc = gb_handle(b, &h_pass)) || (rc = gb_handle(b, &h_it))) return rc;
     if (net && (rc = gb_handle(b, &h_net))) return rc;
+    const PassCtl pc{c, h->opts.rtol, h->opts.inner_rtol, h->opts.max_outer, mixed, h_pass};
+    const PcgCtl ic{c, d, h->opts.max_inner, h_it};
 
     long long l0 = h->nlaunch;
     if ((rc = phys_set_dirichlet(h))) return rc;
@@ -2471,14 +2494,10 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
         if (rk_in && !(h->opts.flags & WPF_SOLVER_FIXED_START)) {
             // the least-squares start: its coefficients need this step's
             // kept residual and level-0 operator, so it is built after them
-            WPF_CUDA(cudaMemsetAsync(d + S_LS0, 0, 6 * sizeof(double), s));
-            WPF_LAUNCH(h, KC_OTHER, k_ctl_ls_begin<<<1, 32, 0, s>>>(c, d, h->opts.rtol,
-                                                                     (long long)g.nx * g.ny * g.nz));
-            WPF_LAUNCH(h, KC_RESID64, k_ws_ls_dots<R><<<row_blocks_for(h, g, k_ws_ls_dots<R>), RB, 0, s>>>(g, L0.cx, L0.cy, L0.cz, L0.diag, h->flags,
-                                                                        h->ws[0], h->ws[1], rk_in, c, 0.0, d));
-            // (the net, when it runs at every solve, needs pass 0's FP32 residual)
-            WPF_LAUNCH(h, KC_OTHER, k_ctl_ws_ls<<<1, 32, 0, s>>>(
-                c, d, (h->opts.flags & WPF_SOLVER_NET_ALWAYS) ? -1.0 : h->opts.rtol));
+            // (the net, when it runs at every solve, needs pass 0's FP32 residual: never skip)
+            WPF_LAUNCH(h, KC_RESID64, k_ws_ls_dots<R><<<row_blocks_for(h, g, k_ws_ls_dots<R>), RB, 0, s>>>(
+                g, L0.cx, L0.cy, L0.cz, L0.diag, h->flags, h->ws[0], h->ws[1], rk_in, c, 0.0,
+                (h->opts.flags & WPF_SOLVER_NET_ALWAYS) ? -1.0 : h->opts.rtol, d));
             WPF_LAUNCH(h, KC_RESID64, k_ws_build_ext<<<rb, RB, 0, s>>>(g, h->ws[0], h->ws[1], 0.f, 0.f, h->ws_e[0],
                                                                        d, &c->wa, dnew));
         } else if (!early) {
@@ -2489,7 +2508,8 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
         const bool lsq = rk_in && !(h->opts.flags & WPF_SOLVER_FIXED_START);
         WPF_LAUNCH(h, KC_RESID64, kern<<<row_blocks_for(h, g, kern), RB, 0, s>>>(
             g, h->pressure, h->T[0], h->T[1], h->T[2], h->flags, h->qterm, resid_dsum(h), L0.cx, L0.cy, L0.cz, L0.diag,
-            h->ws_e[0], H.r, dnew, d, rk_in, lsq ? &c->ls_skip : nullptr));
+            h->ws_e[0], H.r, dnew, d, rk_in, lsq ? &c->ls_skip : nullptr,
+            net ? nullptr : c));
         if (net) {
             // the learned correction in an IF node, taken when the extrapolated
             // start misses rtol by at most NET_WINDOW (k_ctl_net_gate); the
@@ -2517,19 +2537,15 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
             WPF_LAUNCH(h, KC_OTHER, k_ctl_accept_net<<<1, 32, 0, s>>>(c, d));
             WPF_LAUNCH(h, KC_RESID64, k_ws_take_net_dev<R><<<rb, RB, 0, s>>>(
                 g, L0.cx, L0.cy, L0.cz, L0.diag, h->flags, c, h->ws_e[1], H.r, dnew));
-        } else {
-            WPF_LAUNCH(h, KC_OTHER, k_ctl_accept<<<1, 32, 0, s>>>(c, d));
         }
         WPF_LAUNCH(h, KC_RESID64, k_resid64<R><<<row_blocks_for(h, g, k_resid64<R>), RB, 0, s>>>(g, h->pressure, h->T[0], h->T[1], h->T[2],
                                                                    h->flags, h->qterm, resid_dsum(h), H.r, d, 1, &c->accept,
-                                                                   dnew, rk));
+                                                                   dnew, rk, nullptr, pc));
     } else {
         WPF_LAUNCH(h, KC_RESID64, k_resid64<R><<<row_blocks_for(h, g, k_resid64<R>), RB, 0, s>>>(g, h->pressure, h->T[0], h->T[1], h->T[2],
                                                                    h->flags, h->qterm, resid_dsum(h), H.r, d, 1,
-                                                                   nullptr, nullptr, rk));
+                                                                   nullptr, nullptr, rk, nullptr, pc));
     }
-    WPF_LAUNCH(h, KC_OTHER, k_ctl_pass<<<1, 32, 0, s>>>(c, d, h->opts.rtol, h->opts.inner_rtol, h->opts.max_outer,
-                                                         mixed, h_pass));
     if (!net && (rc = gb_join(h))) return rc;   // (with the net it joined before the IF node)
     WPF_CUDA(cudaGetLastError());
     cnt->fixed += h->nlaunch - l0;
@@ -2540,31 +2556,27 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
     if ((rc = gb_begin(pass))) return rc;
     l0 = h->nlaunch;
     WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 4 * sizeof(double), s));   // PQ, RR, RZ0, RZ1
-    WPF_LAUNCH(h, KC_VEC, k_dot<R><<<rb, RB, 0, s>>>(g, H.r, H.r, d + S_RR));
+    WPF_LAUNCH(h, KC_VEC, k_dot<R><<<rb, RB, 0, s>>>(g, H.r, H.r, d + S_RR, ic));
     if (wc) {
         WPF_CUDA(cudaMemsetAsync(d + S_WR, 0, sizeof(double), s));
         WPF_LAUNCH(h, KC_VEC, k_wdot<R><<<rb, RB, 0, s>>>(g, wc, H.r, c, d + S_WR));
         WPF_LAUNCH(h, KC_VEC, k_defl_start<R><<<rb, RB, 0, s>>>(g, wc, h->ws_e[2], c, d, H.x, H.r));
     }
-    WPF_LAUNCH(h, KC_OTHER, k_ctl_pcg_start<<<1, 32, 0, s>>>(c, d, h_it));
     WPF_CUDA(cudaGetLastError());
     if ((rc = gb_end(pass))) return rc;
     if ((rc = gb_cond(pass, cudaGraphCondTypeWhile, h_it, &iter))) return rc;
     if ((rc = gb_begin(iter))) return rc;
     const long long l1 = h->nlaunch;
-    WPF_CUDA(cudaMemsetAsync(d + S_RZ1, 0, sizeof(double), s));
     vcycle(h, H, nu, d + S_RZ1);
     if (wc) {
         WPF_CUDA(cudaMemsetAsync(d + S_WQ, 0, sizeof(double), s));
         WPF_LAUNCH(h, KC_VEC, k_wdot<R><<<rb, RB, 0, s>>>(g, h->ws_e[2], H.z, c, d + S_WQ));
         WPF_LAUNCH(h, KC_OTHER, k_cc_mu<<<1, 32, 0, s>>>(c, d));
     }
-    WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 2 * sizeof(double), s));   // PQ, RR
     launch_apply<R>(h, g, s, L0.cx, L0.cy, L0.cz, L0.diag, H.z, H.p2, H.p, H.q,
                     d + S_RZ1, d + S_RZ0, 0, &c->it, d + S_PQ, wc, d + S_GAM);
     WPF_LAUNCH(h, KC_VEC, k_update_xr<R><<<rb, RB, 0, s>>>(g, H.x, H.r, H.p, H.p2, H.q, d + S_RZ1, d + S_PQ, 0,
-                                                           &c->it, d + S_RR, wc != nullptr));
-    WPF_LAUNCH(h, KC_OTHER, k_ctl_pcg_check<<<1, 32, 0, s>>>(c, d, h->opts.max_inner, h_it));
+                                                           &c->it, d + S_RR, wc != nullptr, ic));
     WPF_CUDA(cudaGetLastError());
     cnt->per_iter = h->nlaunch - l1;
     if ((rc = gb_end(iter))) return rc;
@@ -2572,15 +2584,12 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
     const long long l2 = h->nlaunch;
     WPF_LAUNCH(h, KC_VEC, k_add_correction_dev<R><<<rb, RB, 0, s>>>(g, h->pressure, H.x,
                                                                     ws_on ? h->ws_e[0] : nullptr,
-                                                                    net ? h->ws_e[1] : nullptr, dnew, c));
-    WPF_LAUNCH(h, KC_OTHER, k_ctl_advance<<<1, 32, 0, s>>>(c, d));
+                                                                    net ? h->ws_e[1] : nullptr, dnew, c, d));
     // ||b|| again only after a pass 0 whose residual the least-squares
     // prediction replaced (its ||b|| was the last step's)
     WPF_LAUNCH(h, KC_RESID64, k_resid64<R><<<row_blocks_for(h, g, k_resid64<R>), RB, 0, s>>>(g, h->pressure, h->T[0], h->T[1], h->T[2],
                                                                h->flags, h->qterm, resid_dsum(h), H.r, d, 0,
-                                                               nullptr, nullptr, rk, &c->ls_skip));
-    WPF_LAUNCH(h, KC_OTHER, k_ctl_pass<<<1, 32, 0, s>>>(c, d, h->opts.rtol, h->opts.inner_rtol, h->opts.max_outer,
-                                                         mixed, h_pass));
+                                                               nullptr, nullptr, rk, &c->ls_skip, pc));
     WPF_CUDA(cudaGetLastError());
     cnt->per_pass = (l1 - l0) + (h->nlaunch - l2);
     if ((rc = gb_end(pass))) return rc;
