@@ -1742,9 +1742,20 @@ static void launch_sweep(wpf_handle* h, Hierarchy<R>& H, int l, int cls, bool ze
             g, L.cx, L.cy, L.cz, L.idiag, L.b, in, out, c0, dot, m, err, szc));
 }
 
-// Levels of at most this many cells (FP32 / FP64) run a plain V-cycle.
+// Levels of at most this many cells run a plain V-cycle: the second visit to a
+// level costs launch time of k_coarse in every iteration and saves iterations
+// where a solve takes many.  FP64 from a cold start to 1e-10, three realisations
+// (iterations, ms) with 512 / 2048 / 4096: 40x36x28 41 5.58 / 44 4.93 / 44 4.93,
+// 80x60x50 41 10.1 / 44 8.86 / 55 9.04, 96x80x72 43 13.0 / 47 11.9 / 47 11.9,
+// 64^3 44 7.78 / 44 7.74 / 57 8.47.  FP32 with 1024 / 2048 / 4096: 64^3 44 4.68 /
+// 44 4.67 / 63 5.57, 100x90x110 44 8.85 / 44 8.84 / 63 10.6, 96x80x72 45 7.18 /
+// 49 6.64 / 49 6.59, 128^3 45 11.5 / 45 11.4 / 50 11.3.  A step's solve from an
+// extrapolated FP32 start takes one to three iterations, which the second visit
+// does not save: 128^3, two a step, 718 us with 4096, 750 with 2048.
 template <typename R>
-constexpr long long vcycle_cells() { return sizeof(R) == 4 ? 4096 : 512; }
+static long long vcycle_cells(const wpf_handle* h) {
+    return sizeof(R) == 4 && (h->opts.flags & WPF_SOLVER_EXTRAPOLATE) ? 4096 : 2048;
+}
 
 // The levels that k_coarse takes: from the finest one that fits its shared
 // memory (with cells < COARSE_TOP) down.  Per preconditioner cycle, launches on
@@ -1764,7 +1775,7 @@ template <typename R>
 static CoarsePlan<R> coarse_plan(const wpf_handle* h, const Hierarchy<R>& H, int nu, long long big, int wfrom) {
     CoarsePlan<R> p;
     int lb = H.nlev - 1;   // first level of the plain V-cycle
-    while (lb > 0 && ncells(H.lv[lb - 1].g) <= vcycle_cells<R>()) --lb;
+    while (lb > 0 && ncells(H.lv[lb - 1].g) <= vcycle_cells<R>(h)) --lb;
     unsigned wmask = 0;
     for (int l = 0; l < lb; ++l)
         if (l >= wfrom && ncells(H.lv[l].g) < big) wmask |= 1u << l;
