@@ -28,6 +28,8 @@
 #include "wpf_diag.cuh"
 #include "wpf_internal.cuh"
 
+#include <type_traits>
+
 namespace wpf {
 
 __device__ __forceinline__ long long bits(double v) { return __double_as_longlong(v); }
@@ -740,9 +742,13 @@ __global__ void __launch_bounds__(RB) k_update_split(Grid g, const double* __res
 // concent_rate_lo and the guard-free interface cells phase_cell_lo, at three
 // blocks per SM (80 registers); the plain FP64 form keeps every rate in FP64.
 // PART: 1 the interface cells (the front of the list), 2 the
-// concentration-only cells (the back), 0 both.  The two lists run as two
+// concentration-only cells (the back).  The two lists run as two
 // launches: the concentration-only kernel, without the phase-rate code, fits
 // five blocks per SM (48 registers, no spills) to hide its gathers' latency.
+// A cell that phase_cell_lo refuses waits in the block's queue until there are
+// enough for full warps: the FP64 pipe, which bounds the interface kernel, takes
+// as long for one active lane as for 32, and the refused cells are scattered
+// among the others (18 of 32 lanes active, 150x83x61 late in its run).
 template <bool LOWC, int PART>
 __global__ void __launch_bounds__(RB, PART == 2 ? 5 : (LOWC ? 3 : 0)) k_update_active(Grid g, const Phys* __restrict__ Pp,
                                                       const double* __restrict__ ph,
@@ -766,12 +772,12 @@ __global__ void __launch_bounds__(RB, PART == 2 ? 5 : (LOWC ? 3 : 0)) k_update_a
     int overs = 0;
     const long long sy = g.P, sz = g.S;
     const long long cap = (long long)g.nx * g.ny * g.nz;
-    const int na = nwork[0], nw = na + nwork[1];
-    const int qa = PART == 2 ? na : 0, qb = PART == 1 ? na : nw;
-    for (int q = qa + blockIdx.x * RB + threadIdx.x; q < qb; q += gridDim.x * RB) {
-        // from the back: uniform phase, concentration only
-        const bool uni = PART == 2 ? true : (PART == 1 ? false : q >= na);
-        const long long n = uni ? work[cap - 1 - (q - na)] : work[q];
+    const int na = nwork[0], nb = nwork[1];
+    // One cell; form 0: concentration only, 1: phase_cell_lo (false, nothing
+    // written, where it refuses the cell), 2: phase_cell.
+    auto update = [&](long long n, auto form) -> bool {
+        constexpr int FORM = decltype(form)::value;
+        constexpr bool uni = FORM == 0;
         const long long r = n - XOFF;
         const int k = (int)(r / g.S);
         const long long r2 = r - (long long)k * g.S;
@@ -801,11 +807,12 @@ __global__ void __launch_bounds__(RB, PART == 2 ? 5 : (LOWC ? 3 : 0)) k_update_a
         float rate_lo = 0.f;
         FaceVelF uf{};
         bool have_uf = false;
-        if (!uni) {
-            if (LOWC) lo = phase_cell_lo(ph, n, sy, sz, pr, Tvx, Tvy, Tvz, conc, well, P, K, rate_lo, kxx, over,
-                                         uf, have_uf);
-            if (lo) rate = f32_to_f64(rate_lo);
-            else phase_cell(ph, n, sy, sz, vel, conc, well, P, rate, kxx, over);
+        if constexpr (FORM == 1) {
+            lo = phase_cell_lo(ph, n, sy, sz, pr, Tvx, Tvy, Tvz, conc, well, P, K, rate_lo, kxx, over, uf, have_uf);
+            if (!lo) return false;
+            rate = f32_to_f64(rate_lo);
+        } else if constexpr (FORM == 2) {
+            phase_cell(ph, n, sy, sz, vel, conc, well, P, rate, kxx, over);
         }
         double crate;
         if (well) crate = 0.0;
@@ -834,6 +841,41 @@ __global__ void __launch_bounds__(RB, PART == 2 ? 5 : (LOWC ? 3 : 0)) k_update_a
         if (have_uf) fold_umax_lo(umax, uf);
         kmax = fmax(kmax, kxx);
         overs += over;
+        return true;
+    };
+    if constexpr (PART == 2) {
+        for (int q = blockIdx.x * RB + threadIdx.x; q < nb; q += gridDim.x * RB)
+            update(work[cap - 1 - q], std::integral_constant<int, 0>{});
+    } else if constexpr (!LOWC) {
+        for (int q = blockIdx.x * RB + threadIdx.x; q < na; q += gridDim.x * RB)
+            update(work[q], std::integral_constant<int, 2>{});
+    } else {
+        __shared__ int queue[2 * RB], qn;
+        if (threadIdx.x == 0) qn = 0;
+        __syncthreads();
+        for (int q0 = blockIdx.x * RB; q0 < na; q0 += gridDim.x * RB) {   // block-uniform
+            const int q = q0 + threadIdx.x, lane = threadIdx.x & 31;
+            int refused = -1;
+            if (q < na) {
+                const int n = work[q];
+                if (!update(n, std::integral_constant<int, 1>{})) refused = n;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, refused >= 0);
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&qn, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (refused >= 0) queue[base + __popc(m & ((1u << lane) - 1))] = refused;
+            __syncthreads();
+            const int have = qn;
+            const int n = have >= RB ? queue[have - RB + threadIdx.x] : -1;
+            __syncthreads();
+            if (have < RB) continue;
+            if (threadIdx.x == 0) qn = have - RB;
+            update(n, std::integral_constant<int, 2>{});
+            __syncthreads();
+        }
+        const int have = qn;   // (the loop ends behind a barrier)
+        if (threadIdx.x < have) update(queue[threadIdx.x], std::integral_constant<int, 2>{});
     }
     flush_step_reductions(kmax, P.tau_num, overs, __longlong_as_double((long long)umax), dsc);
 }
