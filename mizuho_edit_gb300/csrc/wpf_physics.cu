@@ -413,19 +413,8 @@ __device__ __forceinline__ void flush_step_reductions(double kmax, double tau_nu
 // (T_new - T_old)(p_b - p_a) to the residual of a live cell a (and the mirror
 // term to b), so that rk becomes the residual under the new T without a pass
 // over the grid (the update changes the phase of a few per cent of the cells).
-// Returns the owner cell a's share (summed by the caller into one atomic) and
-// adds the neighbour's share to rk[b].
-__device__ __forceinline__ double resid_face_delta(double* rk, const uint8_t* __restrict__ fl,
-                                                   const double* __restrict__ pr, long long a, long long b,
-                                                   double p_a, double dT) {
-    if (zero_bits(dT)) return 0.0;   // dT == 0 on the integer pipe
-    const double d = dT * (pr[b] - p_a);
-    if (!(fl[b] & F_DIR)) atomicAdd(rk + b, -d);
-    return d;
-}
-
 constexpr int PB_X = 32, PB_Y = 4, PB_Z = 2;   // k_permeability's block
-__global__ void __launch_bounds__(PB_X * PB_Y * PB_Z) k_permeability(Grid g, Phys P, const double* __restrict__ ph,
+__global__ void __launch_bounds__(PB_X * PB_Y * PB_Z, 8) k_permeability(Grid g, Phys P, const double* __restrict__ ph,
                                const double* __restrict__ prev, const double* __restrict__ kr,
                                double* __restrict__ Tx, double* __restrict__ Ty,
                                double* __restrict__ Tz, double* __restrict__ Kx,
@@ -437,14 +426,24 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z) k_permeability(Grid g, Phy
     // A block of PB_X x PB_Y x PB_Z face-cells; the cell permeabilities its
     // faces need (its cells and the +x/+y/+z neighbours) are computed once
     // each into shared memory instead of once per adjacent face.
+    // The faces to recompute and the cells they need are then listed, so that full
+    // warps take them: the FP64 pipe takes as long for one active lane as for 32,
+    // and late in a run 14 of 32 lanes were active.  256^3 late 592 -> 390 us,
+    // 128^3 early 71 -> 50, 150x83x61 late 55 -> 43.  Blocks of 32x4x2 (256^3, us):
+    // 32x2x2 407, 32x4x4 449, 32x8x2 458; not held to 32 registers 417.
+    constexpr int NT = PB_X * PB_Y * PB_Z;
     constexpr int KX = PB_X + 1, KY = PB_Y + 1, KZ = PB_Z + 1, KN = KX * KY * KZ;
+    static_assert(PB_X == 32 && (PB_Y & (PB_Y - 1)) == 0, "lane = x; rows by masks");
     __shared__ double sK[KN];
     __shared__ unsigned char need[KN];
+    __shared__ unsigned short cells[KN], faces[3 * NT];   // faces: direction * NT + thread of the owner
+    __shared__ int ncells, nfaces;
     const int tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
     const int tid = tx + PB_X * (ty + PB_Y * tz);
     const int i0 = blockIdx.x * PB_X, j0 = blockIdx.y * PB_Y, k0 = blockIdx.z * PB_Z;
     const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
-    for (int q = tid; q < KN; q += PB_X * PB_Y * PB_Z) need[q] = 0;
+    for (int q = tid; q < KN; q += NT) need[q] = 0;
+    if (tid == 0) ncells = nfaces = 0;
     __syncthreads();
     const bool in = i <= g.nx && j <= g.ny && k <= g.nz;
     const long long n = in ? g.at(i, j, k) : 0;
@@ -465,41 +464,69 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z) k_permeability(Grid g, Phy
         if (fz) need[t0 + KX * KY] = 1;
     }
     if (!__syncthreads_or(fx || fy || fz)) return;   // block-uniform
-    for (int q = tid; q < KN; q += PB_X * PB_Y * PB_Z) {
-        if (!need[q]) continue;
-        const int qx = q % KX, qy = (q / KX) % KY, qz = q / (KX * KY);
-        const long long m = g.at(i0 + qx, j0 + qy, k0 + qz);
-        const double f = 0.5 * (1.0 + ph[m]);
-        sK[q] = P.kwh * f + kr[m] * (1.0 - f);   // K0 of :567-574
+    {
+        const unsigned mx = __ballot_sync(0xffffffffu, fx), my = __ballot_sync(0xffffffffu, fy);
+        const unsigned mz = __ballot_sync(0xffffffffu, fz), below = (1u << tx) - 1;
+        int at = 0;
+        if (tx == 0 && (mx | my | mz)) at = atomicAdd(&nfaces, __popc(mx) + __popc(my) + __popc(mz));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (fx) faces[at + __popc(mx & below)] = (unsigned short)tid;
+        at += __popc(mx);
+        if (fy) faces[at + __popc(my & below)] = (unsigned short)(NT + tid);
+        at += __popc(my);
+        if (fz) faces[at + __popc(mz & below)] = (unsigned short)(2 * NT + tid);
+    }
+    for (int q0 = 0; q0 < KN; q0 += NT) {
+        const int q = q0 + tid;
+        const bool on = q < KN && need[q];
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        int at = 0;
+        if (tx == 0 && m) at = atomicAdd(&ncells, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (on) cells[at + __popc(m & ((1u << tx) - 1))] = (unsigned short)q;
     }
     __syncthreads();
-    if (!(fx || fy || fz)) return;   // no barrier below
-    const double a = sK[t0];
-    const double a2 = 2.0 * a;   // 2 a b = (2 a) b exactly: one multiply per face
-    const bool in_j = j >= 1 && j <= g.ny, in_k = k >= 1 && k <= g.nz, in_i = i >= 1 && i <= g.nx;
-    const double p_a = rk ? pr[n] : 0.0;
-    double own = 0.0;
-    // face towards m (owner n; its K0 at tile offset dm): T = 2 a b / (a + b)
-    // / mu, 0 outside `inside`
-    auto face = [&](long long m, int dm, bool inside, double* __restrict__ T, double* __restrict__ Kf,
-                    double* __restrict__ Tv) {
-        const double b = sK[t0 + dm];
-        const double kf = (a2 * b) * rcp_nr(a + b);
-        const double t = inside ? kf * inv_mu : 0.0;
-        if (rk) own += resid_face_delta(rk, fl, pr, n, m, p_a, t - T[n]);
-        T[n] = t;
-        if (Tv) Tv[n] = t * P.inv_dx;
+    const int nk = ncells, nf = nfaces;
+    for (int c = tid; c < nk; c += NT) {
+        const int q = cells[c], qx = q % KX, qy = (q / KX) % KY, qz = q / (KX * KY);
+        const long long m = g.at(i0 + qx, j0 + qy, k0 + qz);
+        const double v = ph[m];   // K0 of :567-574: f = (1 + phase)/2, 1 - f = (1 - phase)/2
+        sK[q] = fma(kr[m], fma(-0.5, v, 0.5), P.kwh * fma(0.5, v, 0.5));
+    }
+    __syncthreads();
+    // face dir of its owner n towards m: T = 2 a b / (a + b) / mu, 0 on the boundary
+    for (int c = tid; c < nf; c += NT) {
+        const int e = faces[c], dir = e / NT, o = e - dir * NT;
+        const int ox = o % PB_X, oy = (o / PB_X) % PB_Y, oz = o / (PB_X * PB_Y);
+        const int fi = i0 + ox, fj = j0 + oy, fk = k0 + oz;
+        const long long a_ = g.at(fi, fj, fk), m = a_ + (dir == 0 ? 1 : (dir == 1 ? g.P : g.S));
+        const int ta = ox + KX * (oy + KY * oz);
+        const double a = sK[ta], b = sK[ta + (dir == 0 ? 1 : (dir == 1 ? KX : KX * KY))];
+        // inside: all three coordinates of the owner, and m's along dir
+        const bool inside = fi >= 1 && fj >= 1 && fk >= 1 && fi <= g.nx - (dir == 0) && fj <= g.ny - (dir == 1) &&
+                            fk <= g.nz - (dir == 2);
+        double* const T = dir == 0 ? Tx : (dir == 1 ? Ty : Tz);
+        double* const Tv = dir == 0 ? Tvx : (dir == 1 ? Tvy : Tvz);
+        double* const Kf = dir == 0 ? Kx : (dir == 1 ? Ky : Kz);
+        const double a2 = 2.0 * a, r = rcp_nr(a + b);   // 2 a b = (2 a) b exactly
+        const double t = inside ? (a2 * inv_mu * b) * r : 0.0;
+        // boundary faces stay 0 (dT = 0): only interior pairs change the residual
+        if (rk) {
+            const double dT = t - T[a_];
+            if (!zero_bits(dT)) {
+                const double d = dT * (pr[m] - pr[a_]);
+                if (!(fl[a_] & F_DIR)) atomicAdd(rk + a_, d);
+                if (!(fl[m] & F_DIR)) atomicAdd(rk + m, -d);
+            }
+        }
+        T[a_] = t;
+        if (Tv) Tv[a_] = t * P.inv_dx;
         if (mark) {   // both cells' level-0 rows use this face
-            mark[n] = 1;
+            mark[a_] = 1;
             mark[m] = 1;
         }
-        if (Kf) Kf[n] = kf;
-    };
-    if (fx) face(n + 1, 1, i >= 1 && i < g.nx && in_j && in_k, Tx, Kx, Tvx);
-    if (fy) face(n + g.P, KX, j >= 1 && j < g.ny && in_i && in_k, Ty, Ky, Tvy);
-    if (fz) face(n + g.S, KX * KY, k >= 1 && k < g.nz && in_i && in_j, Tz, Kz, Tvz);
-    // boundary faces stay 0 (dT = 0): only interior pairs change the residual
-    if (rk && own != 0.0 && !(fl[n] & F_DIR)) atomicAdd(rk + n, own);
+        if (Kf) Kf[a_] = (a2 * b) * r;
+    }
 }
 
 // K0 over every cell of the halo grid (:567-574), for downloads only.
