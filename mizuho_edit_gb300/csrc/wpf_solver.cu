@@ -260,9 +260,10 @@ __global__ void __launch_bounds__(RB) k_resid64(Grid g, const double* __restrict
         else rr += r * r;
     }
     rr += (double)rrr;
-    block_add(rr, dsc + S_RR64);
-    if (want_b) block_add(bb, dsc + S_BB64);
-    if (pc.c && threadIdx.x == 0 && last_block(pc.c)) ctl_pass(pc, dsc);
+    block_adds<2>({rr, bb}, {dsc + S_RR64, want_b ? dsc + S_BB64 : nullptr});
+    if (!pc.c) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(pc.c)) ctl_pass(pc, dsc);
 }
 
 // p += e on the interior (e is zero on dead cells).
@@ -303,8 +304,7 @@ __global__ void __launch_bounds__(RB) k_ws_build_ext(Grid g, const float* __rest
         const float dd = v1 - v2;
         q2 = __fmaf_rn(dd, dd, q2);
     }
-    block_add((double)s2, dsc + S_WSS2);
-    block_add((double)q2, dsc + S_WSD2);
+    block_adds<2>({s2, q2}, {dsc + S_WSS2, dsc + S_WSD2});
 }
 
 template <typename R>
@@ -387,13 +387,11 @@ __global__ void __launch_bounds__(RB) k_ws_ls_dots(Grid g, const R* __restrict__
         bb = fmaf(v, v, bb);
         rr = fmaf(r, r, rr);
     }
-    block_add((double)ra, dsc + S_LS0);
-    block_add((double)rb, dsc + S_LS0 + 1);
-    block_add((double)aa, dsc + S_LS0 + 2);
-    block_add((double)ab, dsc + S_LS0 + 3);
-    block_add((double)bb, dsc + S_LS0 + 4);
-    block_add((double)rr, dsc + S_LS0 + 5);
-    if (c && threadIdx.x == 0 && last_block(c)) ctl_ws_ls(c, dsc, rtol);
+    double* const m = dsc + S_LS0;
+    block_adds<6>({ra, rb, aa, ab, bb, rr}, {m, m + 1, m + 2, m + 3, m + 4, m + 5});
+    if (!c) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(c)) ctl_ws_ls(c, dsc, rtol);
 }
 
 // Pass-0 residual of the start p + e_ext: r0 = r(p) in FP64 exactly as
@@ -495,10 +493,10 @@ __global__ void __launch_bounds__(RB) k_resid64_ws(Grid g, const double* __restr
     }
     rr1 += (double)rr1r;
     rr0 += (double)rr0f;
-    block_add(rr1, dsc + S_RR64);
-    block_add(rr0, dsc + S_RR0WS);
-    block_add(bb, dsc + S_BB64);
-    if (c && threadIdx.x == 0 && last_block(c)) ctl_accept(c, dsc);
+    block_adds<3>({rr1, rr0, bb}, {dsc + S_RR64, dsc + S_RR0WS, dsc + S_BB64});
+    if (!c) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(c)) ctl_accept(c, dsc);
 }
 
 // Accept the learned correction with step alpha: r -= alpha A'e_net,
@@ -541,9 +539,7 @@ __global__ void __launch_bounds__(RB) k_net_dots(Grid g, const R* __restrict__ c
         ww += w * w;
         waw += (R)e2[n] * w;
     }
-    block_add((double)rw, dsc + S_RW);
-    block_add((double)ww, dsc + S_WW);
-    block_add((double)waw, dsc + S_WAW);   // the learned coarse space's operator
+    block_adds<3>({rw, ww, waw}, {dsc + S_RW, dsc + S_WW, dsc + S_WAW});   // (WAW: the learned coarse space's operator)
 }
 
 // p += e (e1 [+ alpha e2]: the accepted start, added once, when e1 != null)
