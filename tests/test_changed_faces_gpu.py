@@ -1,6 +1,8 @@
 """calcPermeability lists the changed faces of a block of 32 x 4 x 2 cells and
 the cells that they need: steps at extents around the block's, from a rough
-state (nearly every face changes) and a smooth one (few do), follow the oracle."""
+state (nearly every face changes) and a smooth one (few do), follow the oracle.
+So does the update's classification, which takes two cells of a row per thread:
+odd, even and short rows."""
 import pytest
 
 from conftest import rel_l2
