@@ -415,9 +415,10 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z, 8) k_permeability(Grid g, 
     // each into shared memory instead of once per adjacent face.
     // The faces to recompute and the cells they need are then listed, so that full
     // warps take them: the FP64 pipe takes as long for one active lane as for 32,
-    // and late in a run 14 of 32 lanes were active.  256^3 late 592 -> 390 us,
-    // 128^3 early 71 -> 50, 150x83x61 late 55 -> 43.  Blocks of 32x4x2 (256^3, us):
-    // 32x2x2 407, 32x4x4 449, 32x8x2 458; not held to 32 registers 417.
+    // and late in a run 14 of 32 lanes were active: 256^3 late 592 -> 390 us, with
+    // ten FP64 instructions a face and three a cell instead of twelve and four
+    // 334; 128^3 early 71 -> 45, 150x83x61 late 55 -> 36.  Blocks of 32x4x2 (256^3,
+    // 390 us): 32x2x2 407, 32x4x4 449, 32x8x2 458; not held to 32 registers 417.
     constexpr int NT = PB_X * PB_Y * PB_Z;
     constexpr int KX = PB_X + 1, KY = PB_Y + 1, KZ = PB_Z + 1, KN = KX * KY * KZ;
     static_assert(PB_X == 32 && (PB_Y & (PB_Y - 1)) == 0, "lane = x; rows by masks");
@@ -474,14 +475,18 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z, 8) k_permeability(Grid g, 
     }
     __syncthreads();
     const int nk = ncells, nf = nfaces;
+    // the harmonic mean is homogeneous: from 2 K0 / mu it gives T = K_f / mu itself,
+    // 2ab/(a+b) = (2a 2b) / (2a + 2b); from 2 K0 where K_f is wanted too
+    const double sc = Kx ? 1.0 : inv_mu, kw = P.kwh * sc;
     for (int c = tid; c < nk; c += NT) {
         const int q = cells[c], qx = q % KX, qy = (q / KX) % KY, qz = q / (KX * KY);
         const long long m = g.at(i0 + qx, j0 + qy, k0 + qz);
-        const double v = ph[m];   // K0 of :567-574: f = (1 + phase)/2, 1 - f = (1 - phase)/2
-        sK[q] = fma(kr[m], fma(-0.5, v, 0.5), P.kwh * fma(0.5, v, 0.5));
+        // 2 K0 / mu, K0 of :567-574: 2 f = 1 + phase, 2 (1 - f) = 1 - phase
+        const double v = ph[m];
+        sK[q] = fma(kr[m], fma(-sc, v, sc), fma(kw, v, kw));
     }
     __syncthreads();
-    // face dir of its owner n towards m: T = 2 a b / (a + b) / mu, 0 on the boundary
+    // face dir of its owner a_ towards m: T = 2 K K' / (K + K') / mu, 0 on the boundary
     for (int c = tid; c < nf; c += NT) {
         const int e = faces[c], dir = e / NT, o = e - dir * NT;
         const int ox = o % PB_X, oy = (o / PB_X) % PB_Y, oz = o / (PB_X * PB_Y);
@@ -495,8 +500,8 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z, 8) k_permeability(Grid g, 
         double* const T = dir == 0 ? Tx : (dir == 1 ? Ty : Tz);
         double* const Tv = dir == 0 ? Tvx : (dir == 1 ? Tvy : Tvz);
         double* const Kf = dir == 0 ? Kx : (dir == 1 ? Ky : Kz);
-        const double a2 = 2.0 * a, r = rcp_nr(a + b);   // 2 a b = (2 a) b exactly
-        const double t = inside ? (a2 * inv_mu * b) * r : 0.0;
+        const double h = (a * b) * rcp_nr(a + b);
+        const double t = inside ? (Kf ? h * inv_mu : h) : 0.0;
         // boundary faces stay 0 (dT = 0): only interior pairs change the residual
         if (rk) {
             const double dT = t - T[a_];
@@ -512,7 +517,7 @@ __global__ void __launch_bounds__(PB_X * PB_Y * PB_Z, 8) k_permeability(Grid g, 
             mark[a_] = 1;
             mark[m] = 1;
         }
-        if (Kf) Kf[a_] = (a2 * b) * r;
+        if (Kf) Kf[a_] = h;
     }
 }
 
@@ -667,13 +672,17 @@ __device__ __forceinline__ void write_halo_of(const Grid& g, int i, int j, int k
 // exactly -1, no acid) stays quiescent for the whole run.  bact_prev = null
 // (after anything else changed the fields) processes every brick.
 //
-// Bound by instructions: a cell's own 26 loads and tests were 500 a warp (256^3
-// late 404 us; the fields' bytes take 55).  A thread now takes two cells of a
-// row, whose tests share the rows beside both: 284 us; 128^3 early 45 -> 34,
-// 150x83x61 late 21 -> 18.  (Held to 48 or 40 registers, 365 and 575 us.  Whole rows by warps with votes: 678 us, a longer
-// serial chain.)
+// Bound by instructions and the chain of a brick: a cell's own 26 loads and tests
+// were 500 instructions a warp (256^3 late 404 us; the fields' bytes take 55).  A
+// thread now takes two cells of a row, whose tests share the rows beside both:
+// 284 us; and a block collects the cells of several bricks in shared memory
+// before it takes its places in the work list, where each brick waited for the
+// answer of two atomics: 260 us.  128^3 early 45 -> 32, 150x83x61 late 21 -> 17.
+// (Held to 48 or 40 registers, 365 and 575 us.  Whole rows by warps with votes: 678
+// us, a longer serial chain.)
 // ---------------------------------------------------------------------------
 constexpr int SPLIT_NT = BRICK_X * BRICK_Y * BRICK_Z / 2;
+constexpr int SPLIT_HOLD = 1024;   // cells a block's list holds before it goes to the work list
 __global__ void __launch_bounds__(SPLIT_NT) k_update_split(Grid g, const double* __restrict__ ph,
                                                            const double* __restrict__ cc,
                                                            const uint8_t* __restrict__ fl,
@@ -689,11 +698,25 @@ __global__ void __launch_bounds__(SPLIT_NT) k_update_split(Grid g, const double*
     const int nbz = (g.nz + BRICK_Z - 1) / BRICK_Z;
     const int nb = nbx * nby * nbz;
     // a thread takes the cells i, i + 1 of a row (i odd: their 16 bytes are aligned)
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const int lx = threadIdx.x % (BRICK_X / 2), row = threadIdx.x / (BRICK_X / 2);
     const int wy = row % BRICK_Y, wz = row / BRICK_Y;
-    constexpr int SPLIT_WARPS = SPLIT_NT / 32;
-    __shared__ int s_cnt[2][SPLIT_WARPS], s_base[2], s_tot[2];
+    __shared__ int list[2][SPLIT_HOLD + BRICK_X * BRICK_Y * BRICK_Z], held[2], base;
+    if (threadIdx.x < 2) held[threadIdx.x] = 0;
+    __syncthreads();
+    // the block's list l (0 interface, 1 concentration-only cells) to the work list
+    auto flush = [&](int l) {
+        const int m = held[l];
+        if (threadIdx.x == 0) base = atomicAdd(nwork + l, m);
+        __syncthreads();
+        const int b0 = base;
+        for (int q = threadIdx.x; q < m; q += SPLIT_NT) {
+            if (l) work[cap - 1 - (b0 + q)] = list[1][q];
+            else work[b0 + q] = list[0][q];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) held[l] = 0;
+    };
     int any_copy = 0;
     for (int t = blockIdx.x; t < nb; t += gridDim.x) {
         const int bx = t % nbx, r = t / nbx, by = r % nby, bz = r / nby;
@@ -774,39 +797,34 @@ __global__ void __launch_bounds__(SPLIT_NT) k_update_split(Grid g, const double*
                 }
             }
         }
-        // one atomic per list and brick: the two counters are the same two
-        // addresses for every block, and atomics on one address serialise
+        // into the block's lists, in the order of the cells, so that the update's
+        // warps read rows
         const unsigned ma0 = __ballot_sync(0xffffffffu, !uni[0]), ma1 = __ballot_sync(0xffffffffu, !uni[1]);   // interface cells
         const unsigned mb0 = __ballot_sync(0xffffffffu, uni[0] && !copy[0]);   // concentration-only cells
         const unsigned mb1 = __ballot_sync(0xffffffffu, uni[1] && !copy[1]);
-        if (lane == 0) {
-            s_cnt[0][warp] = __popc(ma0) + __popc(ma1);
-            s_cnt[1][warp] = __popc(mb0) + __popc(mb1);
-        }
-        __syncthreads();
-        if (threadIdx.x < 2) {
-            int tot = 0;
-            for (int w = 0; w < SPLIT_WARPS; ++w) tot += s_cnt[threadIdx.x][w];
-            s_base[threadIdx.x] = tot ? atomicAdd(nwork + threadIdx.x, tot) : 0;
-            s_tot[threadIdx.x] = tot;
-        }
-        __syncthreads();
-        int offa = s_base[0], offb = s_base[1];
-        for (int w = 0; w < warp; ++w) {
-            offa += s_cnt[0][w];
-            offb += s_cnt[1][w];
-        }
-        // in the order of the cells, so that the update's warps read rows
         const unsigned below = (1u << lane) - 1;
-        offa += __popc(ma0 & below) + __popc(ma1 & below);
-        offb += __popc(mb0 & below) + __popc(mb1 & below);
-        if (!uni[0]) work[offa++] = n;
-        if (!uni[1]) work[offa] = n + 1;
-        if (uni[0] && !copy[0]) work[cap - 1 - offb++] = n;
-        if (uni[1] && !copy[1]) work[cap - 1 - offb] = n + 1;
-        if (threadIdx.x == 0 && bact_cur) bact_cur[t] = (uint8_t)((s_tot[0] + s_tot[1]) > 0);
-        __syncthreads();   // s_cnt / s_tot are rewritten for the next brick
+        if (ma0 | ma1) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&held[0], __popc(ma0) + __popc(ma1));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(ma0 & below) + __popc(ma1 & below);
+            if (!uni[0]) list[0][at++] = n;
+            if (!uni[1]) list[0][at] = n + 1;
+        }
+        if (mb0 | mb1) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&held[1], __popc(mb0) + __popc(mb1));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(mb0 & below) + __popc(mb1 & below);
+            if (uni[0] && !copy[0]) list[1][at++] = n;
+            if (uni[1] && !copy[1]) list[1][at] = n + 1;
+        }
+        const int active = __syncthreads_or(ma0 | ma1 | mb0 | mb1);
+        if (threadIdx.x == 0 && bact_cur) bact_cur[t] = (uint8_t)(active != 0);
+        if (held[0] > SPLIT_HOLD) flush(0);   // (block-uniform: nothing is added before flush's or the next brick's barrier)
+        if (held[1] > SPLIT_HOLD) flush(1);
+        __syncthreads();
     }
+    if (held[0]) flush(0);
+    if (held[1]) flush(1);
     if (__syncthreads_or(any_copy) && threadIdx.x == 0)
         atomicMin(reinterpret_cast<unsigned long long*>(dsc + S_TAUMIN_KEY), dkey(tau0));
 }
