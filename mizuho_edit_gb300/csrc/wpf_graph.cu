@@ -180,13 +180,22 @@ __global__ void k_step_begin(StepCtl* c, double* dsc, double dt_c, double dt_a, 
     dsc[S_WSD2] = 0.0;
 }
 
-// A converged solve's increment becomes the newest of the history.
-__global__ void k_step_end(StepCtl* c) {
-    if (threadIdx.x) return;
-    if (c->status == WPF_OK) {
+// A converged solve's increment becomes the newest of the history; the control
+// block and the slots go to their page-locked host copies, which the kernel
+// reaches itself (two copy nodes took 3 us each).
+constexpr int END_NT = 64;
+static_assert(sizeof(StepCtl) % sizeof(double) == 0 && S_COUNT <= END_NT && sizeof(StepCtl) / sizeof(double) <= END_NT,
+              "one word per thread");
+__global__ void k_step_end(StepCtl* c, const double* dsc, StepCtl* c_host, double* dsc_host) {
+    const int t = threadIdx.x;
+    if (t == 0 && c->status == WPF_OK) {
         c->h2 = c->h1;
         c->h1 = c->dt;
     }
+    __syncthreads();
+    if (t < (int)(sizeof(StepCtl) / sizeof(double)))
+        reinterpret_cast<long long*>(c_host)[t] = reinterpret_cast<const long long*>(c)[t];
+    if (t < S_COUNT) reinterpret_cast<long long*>(dsc_host)[t] = reinterpret_cast<const long long*>(dsc)[t];
 }
 
 // ---- host side ------------------------------------------------------------------
@@ -270,10 +279,8 @@ int step_graph_capture(wpf_handle* h, GraphBuilder& b, StepCounts* n) {
     drop_split(h);
     if (rc) return rc;
     l0 = h->nlaunch;
-    WPF_LAUNCH(h, KC_OTHER, k_step_end<<<1, 32, 0, s>>>(c));
+    WPF_LAUNCH(h, KC_OTHER, k_step_end<<<1, END_NT, 0, s>>>(c, h->dsc, h->gctl_host, h->gdsc_host));
     WPF_CUDA(cudaGetLastError());
-    WPF_CUDA(cudaMemcpyAsync(h->gctl_host, c, sizeof(StepCtl), cudaMemcpyDeviceToHost, s));
-    WPF_CUDA(cudaMemcpyAsync(h->gdsc_host, h->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
     n->fixed += h->nlaunch - l0;
     return gb_end(b);
 }

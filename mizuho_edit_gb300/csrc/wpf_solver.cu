@@ -72,14 +72,23 @@ __device__ __forceinline__ bool last_block(StepCtl* c) {
     return true;
 }
 
-// After a refinement pass's residual (S_RR64, S_BB64): the pass logic of solve_impl.
+// PCG prologue (r.r in S_RR) and the test after an iteration.
+struct PcgCtl {
+    StepCtl* c = nullptr;
+    double* dsc = nullptr;
+    int maxit = 0;
+    cudaGraphConditionalHandle h = 0;
+};
+// After a refinement pass's residual (S_RR64, S_BB64): the pass logic of
+// solve_impl, and with ic the PCG's prologue too (r.r is the residual's).
 struct PassCtl {
     StepCtl* c = nullptr;   // null: none (the host takes the decision)
     double rtol = 0.0, inner_rtol = 0.0;
     int max_outer = 0, mixed = 0;
     cudaGraphConditionalHandle h = 0;
+    PcgCtl ic;
 };
-__device__ __noinline__ void ctl_pass(const PassCtl& a, const double* dsc) {
+__device__ __noinline__ void ctl_pass(const PassCtl& a, double* dsc) {
     StepCtl* c = a.c;
     const double rr = __ldcg(dsc + S_RR64), bb = __ldcg(dsc + S_BB64);
     const int pass = c->pass;
@@ -108,17 +117,20 @@ __device__ __noinline__ void ctl_pass(const PassCtl& a, const double* dsc) {
         }
     }
     c->need_pcg = pcg;
+    if (a.ic.c) {   // (a residual above rtol is not zero: the iterations run)
+        c->it = 0;
+        if (pcg) {
+            ++c->pcgs;
+            c->r0 = sqrt(rr);
+        }
+        dsc[S_PQ] = dsc[S_RR] = dsc[S_RZ0] = dsc[S_RZ1] = 0.0;
+        cudaGraphSetConditional(a.ic.h, pcg);
+    }
     cudaGraphSetConditional(a.h, cont);
 }
 
-// PCG prologue (r.r in S_RR) and the test after an iteration.
-struct PcgCtl {
-    StepCtl* c = nullptr;
-    double* dsc = nullptr;
-    int maxit = 0;
-    cudaGraphConditionalHandle h = 0;
-};
-// The iterations run when the pass needs a PCG and ||r_0|| > 0 (pcg's early return).
+// r.r in S_RR: the iterations run when the pass needs a PCG and ||r_0|| > 0 (pcg's
+// early return).  For a start whose learned correction changed r after its sums.
 __device__ __noinline__ void ctl_pcg_start(const PcgCtl& a) {
     StepCtl* c = a.c;
     int run = 0;
@@ -197,6 +209,9 @@ __device__ __forceinline__ double resid_cell(double q, double p0, double pxp, do
                 typ * (pyp - p0) + tzp * (pzp - p0));
 }
 
+// q == 0 on the integer pipe (an FP64 comparison takes the FP64 pipe's time)
+__device__ __forceinline__ bool zero64(double q) { return (__double_as_longlong(q) << 1) == 0; }
+
 template <typename R>
 __global__ void __launch_bounds__(RB) k_resid64(Grid g, const double* __restrict__ pr,
                                                 const double* __restrict__ Tx,
@@ -239,7 +254,7 @@ __global__ void __launch_bounds__(RB) k_resid64(Grid g, const double* __restrict
             const double pxp = pr[n + 1], pxm = pr[n - 1], pyp = pr[n + sy], pym = pr[n - sy];
             const double pzp = pr[n + sz], pzm = pr[n - sz];
             r = resid_cell(q, p0, pxp, pxm, pyp, pym, pzp, pzm, txp, txm, typ, tym, tzp, tzm, D, n);
-            if (want_b && (q != 0.0 || ((fl[n - sz] | fl[n - sy] | fl[n - 1] | fl[n + 1] |
+            if (want_b && (!zero64(q) || ((fl[n - sz] | fl[n - sy] | fl[n - 1] | fl[n + 1] |
                                          fl[n + sy] | fl[n + sz]) & F_DIR))) {
                 double bref = -q;
                 if (fl[n - sz] & F_DIR) bref -= pzm * tzm;
@@ -458,7 +473,7 @@ __global__ void __launch_bounds__(RB) k_resid64_ws(Grid g, const double* __restr
                 // r(p) kept from the last residual pass, corrected face by
                 // face for the new T: FP64 work only next to a Dirichlet cell
                 r0 = rk_in[n];
-                if (dm || (qterm && q != 0.0))
+                if (dm || !zero64(q))
                     bref_add(pr[n + 1], pr[n - 1], pr[n + sy], pr[n - sy], pr[n + sz], pr[n - sz], Tx[n],
                              Tx[n - 1], Ty[n], Ty[n - sy], Tz[n], Tz[n - sz]);
             } else {
@@ -468,7 +483,7 @@ __global__ void __launch_bounds__(RB) k_resid64_ws(Grid g, const double* __restr
                 const double pxp = pr[n + 1], pxm = pr[n - 1], pyp = pr[n + sy], pym = pr[n - sy];
                 const double pzp = pr[n + sz], pzm = pr[n - sz];
                 r0 = resid_cell(q, p0, pxp, pxm, pyp, pym, pzp, pzm, txp, txm, typ, tym, tzp, tzm, D, n);
-                if (dm || q != 0.0) bref_add(pxp, pxm, pyp, pym, pzp, pzm, txp, txm, typ, tym, tzp, tzm);
+                if (dm || !zero64(q)) bref_add(pxp, pxm, pyp, pym, pzp, pzm, txp, txm, typ, tym, tzp, tzm);
             }
             e = e1[n];
             if (D) {
@@ -2525,8 +2540,8 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
     int rc;
     if ((rc = gb_handle(b, &h_pass)) || (rc = gb_handle(b, &h_it))) return rc;
     if (net && (rc = gb_handle(b, &h_net))) return rc;
-    const PassCtl pc{c, h->opts.rtol, h->opts.inner_rtol, h->opts.max_outer, mixed, h_pass};
     const PcgCtl ic{c, d, h->opts.max_inner, h_it};
+    const PassCtl pc{c, h->opts.rtol, h->opts.inner_rtol, h->opts.max_outer, mixed, h_pass, net ? PcgCtl{} : ic};
 
     long long l0 = h->nlaunch;
     if ((rc = phys_set_dirichlet(h))) return rc;
@@ -2603,17 +2618,19 @@ static int solve_capture_impl(wpf_handle* h, Hierarchy<R>& H, GraphBuilder& b, S
 
     GraphBuilder pass, iter;
     if ((rc = gb_cond(b, cudaGraphCondTypeWhile, h_pass, &pass))) return rc;
-    if ((rc = gb_begin(pass))) return rc;
     l0 = h->nlaunch;
-    WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 4 * sizeof(double), s));   // PQ, RR, RZ0, RZ1
-    WPF_LAUNCH(h, KC_VEC, k_dot<R><<<rb, RB, 0, s>>>(g, H.r, H.r, d + S_RR, ic));
-    if (wc) {
-        WPF_CUDA(cudaMemsetAsync(d + S_WR, 0, sizeof(double), s));
-        WPF_LAUNCH(h, KC_VEC, k_wdot<R><<<rb, RB, 0, s>>>(g, wc, H.r, c, d + S_WR));
-        WPF_LAUNCH(h, KC_VEC, k_defl_start<R><<<rb, RB, 0, s>>>(g, wc, h->ws_e[2], c, d, H.x, H.r));
+    if (net) {   // (else ctl_pass starts the PCG)
+        if ((rc = gb_begin(pass))) return rc;
+        WPF_CUDA(cudaMemsetAsync(d + S_PQ, 0, 4 * sizeof(double), s));   // PQ, RR, RZ0, RZ1
+        WPF_LAUNCH(h, KC_VEC, k_dot<R><<<rb, RB, 0, s>>>(g, H.r, H.r, d + S_RR, ic));
+        if (wc) {
+            WPF_CUDA(cudaMemsetAsync(d + S_WR, 0, sizeof(double), s));
+            WPF_LAUNCH(h, KC_VEC, k_wdot<R><<<rb, RB, 0, s>>>(g, wc, H.r, c, d + S_WR));
+            WPF_LAUNCH(h, KC_VEC, k_defl_start<R><<<rb, RB, 0, s>>>(g, wc, h->ws_e[2], c, d, H.x, H.r));
+        }
+        WPF_CUDA(cudaGetLastError());
+        if ((rc = gb_end(pass))) return rc;
     }
-    WPF_CUDA(cudaGetLastError());
-    if ((rc = gb_end(pass))) return rc;
     if ((rc = gb_cond(pass, cudaGraphCondTypeWhile, h_it, &iter))) return rc;
     if ((rc = gb_begin(iter))) return rc;
     const long long l1 = h->nlaunch;
