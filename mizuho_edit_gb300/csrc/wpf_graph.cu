@@ -4,10 +4,11 @@
 // calcPermeability, solvePressure, the fused velocity/phase/concentration
 // update) reads a scalar back after every residual and every PCG iteration to
 // decide what to launch next.  Here the whole step is one CUDA graph: the dt
-// law and the solver's decisions run in one-thread control kernels, the two
-// solver loops are conditional WHILE nodes whose handles those kernels set,
-// and the step ends with two device-to-host copies (the control block and the
-// scalar slots) read after the one synchronisation of the step.  The kernels
+// law runs in a one-thread kernel, the solver's decisions in the last blocks of
+// the kernels that form their sums, the two solver loops are conditional WHILE
+// nodes whose handles those blocks set, and the step's last kernel writes the
+// control block and the scalar slots to page-locked memory, read after the one
+// synchronisation of the step.  The kernels
 // are those of the host-driven step, so are the results; only the fused
 // update's classification and the extrapolated start's build run on side
 // branches (beside the solve and beside calcPermeability).

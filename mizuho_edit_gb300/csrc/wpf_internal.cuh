@@ -114,7 +114,7 @@ EncodeTiledFn tensor_map_encoder();
 
 // Control block of the device-resident step (WPF_SOLVER_STEP_GRAPH): the
 // decisions the host-driven step takes after each read-back, taken instead by
-// one-thread kernels inside the step graph.  Copied back once per step.
+// the kernels of the step graph.  Copied back once per step.
 struct StepCtl {
     double dt;               // this step's dt (the dt law on the device)
     double h1, h2;           // step sizes of the last two increments
@@ -624,11 +624,29 @@ inline unsigned row_blocks_for(const wpf_handle* h, const Grid& g, F f) {
     return row_blocks(h, g, per_sm);
 }
 
+// *acc += the block's sum of v.  Of doubles (blocks of RB threads) the first warp
+// sums eight a lane from shared memory: 13 FP64 instructions instead of a shuffle
+// tree's 45 at 16 cycles each (96x80x72 FP64: the last half-sweep with r.z 16.1 ->
+// 13.7 us, the residual update 8.6 -> 7.6).
 template <typename T>
 __device__ __forceinline__ void block_add(T v, double* acc) {
-    __shared__ T sm_add[32];
-    v = block_sum(v, sm_add);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) atomicAdd(acc, (double)v);
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    if constexpr (sizeof(T) == 8) {
+        __shared__ T sm_add[RB];
+        __syncthreads();
+        sm_add[tid] = v;
+        __syncthreads();
+        if (tid >= 32) return;
+        T s = 0;
+#pragma unroll
+        for (int u = 0; u < RB / 32; ++u) s += sm_add[tid + 32 * u];
+        s = warp_sum(s);
+        if (tid == 0) atomicAdd(acc, s);
+    } else {
+        __shared__ T sm_add[32];
+        v = block_sum(v, sm_add);
+        if (tid == 0) atomicAdd(acc, (double)v);
+    }
 }
 
 // *acc[q] += the block's sum of v[q], taken in FP64 (acc[q] null: not), in a

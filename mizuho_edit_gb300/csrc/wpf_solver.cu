@@ -23,7 +23,7 @@
 // correction over-relaxed by 2, which makes piecewise-constant interpolation
 // effective); red-black Gauss-Seidel smoothing (symmetric: red-black before,
 // black-red after) so the V-cycle is a symmetric preconditioner; coarsening
-// down to <= 2 cells per axis, solved by Gauss-Seidel sweeps in one block.
+// down to <= 64 cells, solved by Gauss-Seidel half-sweeps in one block.
 // Dead cells (Dirichlet, or aggregates of only Dirichlet cells) carry a zero
 // diagonal and zero couplings and never change.
 //
@@ -2413,8 +2413,8 @@ static int solve_impl(wpf_handle* h, Hierarchy<R>& H, wpf_step_stats* st) {
 // ---------------------------------------------------------------------------
 // Device-resident solve (WPF_SOLVER_STEP_GRAPH).  The same kernels as
 // solve_impl / pcg and the fused update; the decisions those functions take
-// on the host after each read-back are taken by one-thread control kernels,
-// and the two loops are conditional WHILE nodes:
+// on the host after each read-back are taken by the last block of the kernel
+// that forms their sums, and the two loops are conditional WHILE nodes:
 //   [Dirichlet, level-0 coefficients]
 //   { pass-0 residual (extrapolated start + fallback), pass test  ||  coarse levels }
 //   WHILE(passes) { [PCG prologue]  WHILE(iterations) { [cycle, apply, update, test] }

@@ -17,7 +17,7 @@ Why one graph launch per ensemble step rather than one persistent kernel:
 every PCG iteration of every member ends in a reduction that decides the next
 launch, so a persistent kernel would need a grid-wide barrier per solver phase
 of each member and one block shape for kernels whose best shapes differ
-(32x8 sweep tiles, 128-row patches, the one-block bottom cycle); the graph
+(32x8 sweep tiles, 128-row patches, the cluster of the coarse levels); the graph
 keeps each kernel's own launch shape, turns the decisions into conditional
 nodes evaluated on the device and still costs one launch and one
 synchronisation per ensemble step.
