@@ -770,6 +770,8 @@ static int launch_conv_t(const ConvArgs& a, cudaStream_t s) {
 }
 
 static int launch_conv(int cin, int cout, const ConvArgs& a, cudaStream_t s) {
+    // 16-byte copies and stores
+    if ((((uintptr_t)a.in | (uintptr_t)a.w | (uintptr_t)a.out16 | (uintptr_t)a.out32) & 15) != 0) return WPF_ERR_ARG;
 #define WPF_CONV_CASE(I, O) \
     if (cin == I && cout == O) return launch_conv_t<I, O>(a, s);
     WPF_CONV_CASE(16, 16) WPF_CONV_CASE(16, 32) WPF_CONV_CASE(32, 64) WPF_CONV_CASE(64, 64)
@@ -1140,7 +1142,30 @@ int wpf_conv3d_wgrad(int32_t cin, int32_t cout, int32_t nx, int32_t ny, int32_t 
         WPF_CUDA(cudaMalloc((void**)&derr, sizeof(int)));
         WPF_CUDA(cudaMemset(derr, 0, sizeof(int)));
     }
-    int rc = launch_wgrad(cin, cout, nx, ny, nz, x, gy, gw, derr, s);
+    // the kernels copy 16 bytes at a time: an operand on another boundary is copied
+    // first (freed after the synchronisation below)
+    struct Copies {
+        void* p[2] = {nullptr, nullptr};
+        ~Copies() {
+            for (void* q : p)
+                if (q) cudaFree(q);
+        }
+    } tmp;
+    auto aligned = [&](const uint16_t*& src, int channels, void*& copy) -> int {
+        if (((uintptr_t)src & 15) == 0) return WPF_OK;
+        const size_t bytes = (size_t)nx * ny * nz * channels * 2;
+        if (cudaMalloc(&copy, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return WPF_ERR_NOMEM;
+        }
+        WPF_CUDA(cudaMemcpyAsync(copy, src, bytes, cudaMemcpyDeviceToDevice, s));
+        src = (const uint16_t*)copy;
+        return WPF_OK;
+    };
+    int rc = cin < 1 || cout < 1 ? WPF_ERR_ARG : aligned(x, cin, tmp.p[0]);
+    if (!rc) rc = aligned(gy, cout, tmp.p[1]);
+    if (rc) return rc;
+    rc = launch_wgrad(cin, cout, nx, ny, nz, x, gy, gw, derr, s);
     if (rc) return rc;
     if (gb) {
         BiasArgs ba = {};

@@ -51,3 +51,38 @@ def test_conv_and_wgrad_match_oracle(shape, cin, cout):
                                       _ptr(gb), None), "wgrad")
         assert rel_l2(gw.cpu().numpy()[pad:].reshape(cout, 27, cin), gw_ref) < 1e-5
         assert rel_l2(gb.cpu().numpy(), gb_ref) < 1e-5
+
+
+@pytest.mark.parametrize("shift", [1, 4])
+def test_operands_off_16_byte_boundaries(shift):
+    """The weight gradient takes its operands on any boundary; the convolution, whose copies and
+    stores are 16 bytes wide, refuses them."""
+    import torch
+    from mizuho_edit_gb300 import capi
+    L = capi.load()
+    nx, ny, nz, cin, cout = 9, 17, 3, 16, 32
+    rng = np.random.default_rng(shift)
+    x = N.bf16(rng.standard_normal((nz, ny, nx, cin)))
+    gy = N.bf16(rng.standard_normal((nz, ny, nx, cout)))
+
+    def off(a):
+        b = _bits(a).reshape(-1)
+        t = torch.zeros(b.numel() + 16, dtype=b.dtype, device="cuda")
+        t[shift:shift + b.numel()] = b
+        return t, C.c_void_p(t.data_ptr() + 2 * shift)
+
+    (tx, px), (tg, pg) = off(x), off(gy)
+    gw_ref, gb_ref = N.conv3d_wgrad(x, gy)
+    ax, ag = _bits(x), _bits(gy)
+    for qx, qg in ((px, pg), (px, _ptr(ag)), (_ptr(ax), pg)):
+        gw = torch.zeros(cout * 27 * cin, device="cuda")
+        gb = torch.zeros(cout, device="cuda")
+        capi.check(L.wpf_conv3d_wgrad(cin, cout, nx, ny, nz, qx, qg, _ptr(gw), _ptr(gb), None), "wgrad")
+        assert rel_l2(gw.cpu().numpy().reshape(cout, 27, cin), gw_ref) < 1e-5
+        assert rel_l2(gb.cpu().numpy(), gb_ref) < 1e-5
+    w = torch.zeros(cout * 27 * cin + 16, dtype=torch.int16, device="cuda")
+    out = torch.zeros(nz * ny * nx * cout + 16, device="cuda")
+    bad = C.c_void_p(w.data_ptr() + 2 * shift)
+    assert L.wpf_conv3d(cin, cout, nx, ny, nz, px, _ptr(w), None, 0, None, _ptr(out), None) != 0
+    assert L.wpf_conv3d(cin, cout, nx, ny, nz, _ptr(ax), bad, None, 0, None, _ptr(out), None) != 0
+    assert L.wpf_conv3d(cin, cout, nx, ny, nz, _ptr(ax), _ptr(w), None, 0, None, C.c_void_p(out.data_ptr() + 4), None) != 0
