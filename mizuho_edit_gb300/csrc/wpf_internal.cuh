@@ -398,6 +398,23 @@ namespace wpf {
 // release: let the launch after start (both do nothing in an ordinary launch).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launch k programmatically behind the launch before it on s; as an ordinary launch
+// where that one is not a kernel that waits itself, or where event records stand
+// between the two.
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(bool behind, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
 
 // ---- error helpers --------------------------------------------------------
 #define WPF_CUDA(call)                                   \

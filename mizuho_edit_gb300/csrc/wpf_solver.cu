@@ -1931,23 +1931,6 @@ static CoarsePlan<R> coarse_plan(const wpf_handle* h, const Hierarchy<R>& H, int
     return p;
 }
 
-// Launch k programmatically behind the launch before it on s (see k_rbgs); as an
-// ordinary launch where that one is not a kernel of this cycle, or where the
-// timers put event records between the two.
-template <typename... P, typename... A>
-static cudaError_t launch_behind(bool behind, void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = s;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = behind ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
-}
-
 template <typename R>
 static void launch_coarse(wpf_handle* h, CoarsePlan<R>& p, int cls, double* dot, bool behind, cudaStream_t s) {
     p.args.dot = dot;
@@ -1985,7 +1968,7 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& pl
     const bool is_big = ncells(g) >= big;
     const int gamma = (l >= wfrom && !is_big) ? 2 : 1;
     auto restrict_from = [&](const R* x) {
-        WPF_LAUNCH(h, KC_MGREST, launch_behind(pdl, k_resid_restrict<R>, cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), s,
+        WPF_LAUNCH(h, KC_MGREST, launch_behind(pdl, k_resid_restrict<R>, cell_grid(C.g.nx, C.g.ny, C.g.nz), cell_block(), 0, s,
                                                g, C.g, L.cx, L.cy, L.cz, L.diag, L.idiag, x, L.b, C.b));
     };
     if (is_big) {
@@ -2011,15 +1994,15 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& pl
     dim3 hb, hg;
     rbgs_grid<R>(g, hg, hb);
     auto half = [&](int color) {
-        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs<R>, hg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, color));
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs<R>, hg, hb, 0, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, color));
     };
     // (the first launch on level 0 is the cycle's first)
-    WPF_LAUNCH(h, cls, launch_behind(pdl && l > 0, k_rbgs_zero<R>, hg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b));
+    WPF_LAUNCH(h, cls, launch_behind(pdl && l > 0, k_rbgs_zero<R>, hg, hb, 0, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b));
     for (int it = 1; it < nu; ++it) { half(0); half(1); }
     for (int rep = 0; rep < gamma; ++rep) {
         restrict_from(L.x);
         cycle_level(h, H, l + 1, plan, nu, big, wfrom, nullptr);
-        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_corr<R>, hg, hb, s, g, C.g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, C.x));
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_corr<R>, hg, hb, 0, s, g, C.g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, C.x));
         for (int it = 1; it < nu; ++it) { half(0); half(1); }
         if (rep + 1 < gamma) {   // the post-sweeps' last red half-sweep is the pre-sweeps' first
             for (int it = 0; it < nu; ++it) { half(0); half(1); }
@@ -2030,7 +2013,7 @@ static void cycle_level(wpf_handle* h, Hierarchy<R>& H, int l, CoarsePlan<R>& pl
         const long long nz = (long long)h->nsm * 8 / plane;
         dim3 dg = hg;
         dg.z = (unsigned)(nz < 1 ? 1 : (nz < hg.z ? nz : hg.z));
-        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_dot<R>, dg, hb, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, rz));
+        WPF_LAUNCH(h, cls, launch_behind(pdl, k_rbgs_dot<R>, dg, hb, 0, s, g, L.cx, L.cy, L.cz, L.idiag, L.x, L.b, rz));
         return;
     }
     half(0);
