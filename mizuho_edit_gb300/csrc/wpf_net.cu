@@ -566,29 +566,6 @@ struct BiasArgs {
     float* gb[WPF_NET_LAYERS];
     int nvox[WPF_NET_LAYERS], cout[WPF_NET_LAYERS];
 };
-__global__ void k_bias_grad(BiasArgs a) {
-    pdl_wait();
-    pdl_release();
-    __shared__ float s[64];
-    if (threadIdx.x < 64) s[threadIdx.x] = 0.f;
-    __syncthreads();
-    const int l = blockIdx.y, cout = a.cout[l], nvox = a.nvox[l];
-    const bf16_t* __restrict__ gy = a.gy[l];
-    const int co = threadIdx.x % cout;
-    const int lanes = blockDim.x / cout;
-    float acc = 0.f;
-    for (long long v = (long long)blockIdx.x * lanes + threadIdx.x / cout; v < nvox;
-         v += (long long)gridDim.x * lanes)
-        acc += bf2f(gy[v * cout + co]);
-    atomicAdd(&s[co], acc);
-    __syncthreads();
-    if (threadIdx.x < cout) atomicAdd(&a.gb[l][threadIdx.x], s[threadIdx.x]);
-}
-
-// ---- elementwise pieces of the U-Net ----------------------------------------------
-// out = 2x2x2 mean of in (dims of in: nx, ny, nz, even)
-// One thread per (coarse voxel, 8-channel chunk): 16-byte loads and stores.
-// Per channel the same sum in the same order as the element-wise form.
 __device__ __forceinline__ void unpack8(const uint4 q, float* f) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -597,34 +574,69 @@ __device__ __forceinline__ void unpack8(const uint4 q, float* f) {
         f[2 * i + 1] = bf2f((bf16_t)(w[i] >> 16));
     }
 }
+// A thread takes eight channels of a voxel (16-byte loads).
+__global__ void k_bias_grad(BiasArgs a) {
+    __shared__ float s[64];
+    if (threadIdx.x < 64) s[threadIdx.x] = 0.f;
+    __syncthreads();
+    pdl_wait();
+    pdl_release();
+    const int l = blockIdx.y, cout = a.cout[l], nvox = a.nvox[l];
+    const bf16_t* __restrict__ gy = a.gy[l];
+    const int per = cout / 8, c = threadIdx.x % per * 8, lanes = blockDim.x / per;
+    float acc[8] = {};
+#pragma unroll 4
+    for (long long v = (long long)blockIdx.x * lanes + threadIdx.x / per; v < nvox;
+         v += (long long)gridDim.x * lanes) {
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4*>(gy + v * cout + c), f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {   // lanes `per` apart hold the same channels
+        for (int o = 16; o >= per; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+        if ((int)(threadIdx.x & 31) < per) atomicAdd(&s[c + e], acc[e]);
+    }
+    __syncthreads();
+    if (threadIdx.x < cout) atomicAdd(&a.gb[l][threadIdx.x], s[threadIdx.x]);
+}
 
+// ---- elementwise pieces of the U-Net ----------------------------------------------
+// out = 2x2x2 mean of in (dims of in: nx, ny, nz, even)
+// One thread per (coarse voxel, 8-channel chunk): 16-byte loads and stores.
+// Per channel the same sum in the same order as the element-wise form.
+// Places are a chunk and a voxel of 32 bits: 64-bit divisions were most of the
+// instructions.  Backward and bias kernels moved single elements before: training
+// step 48x40x32 393 -> 384 us a call.
+__device__ __forceinline__ uint4 pack8(const float* f) {
+    return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+}
 __global__ void k_pool2(const bf16_t* __restrict__ in, bf16_t* __restrict__ out, int nx, int ny, int nz,
                         int C) {
     pdl_wait();
     pdl_release();
-    const int hx = nx / 2, hy = ny / 2, hz = nz / 2, C8 = C / 8;
-    const long long n = (long long)hx * hy * hz * C8;
+    const int hx = nx / 2, hy = ny / 2, hz = nz / 2, sh = __ffs(C) - 4, C8 = 1 << sh;   // (C: 16, 32 or 64)
+    const long long n = (long long)hx * hy * hz << sh;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
          q += (long long)gridDim.x * blockDim.x) {
-        const int c8 = (int)(q % C8);
-        long long V = q / C8;
-        const int X = (int)(V % hx);
-        V /= hx;
-        const int Y = (int)(V % hy), Z = (int)(V / hy);
+        const int c8 = (int)q & (C8 - 1);
+        const unsigned V = (unsigned)(q >> sh), R = V / hx;
+        const int X = V - R * hx, Z = R / hy, Y = R - Z * hy;
         float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int k = 0; k < 2; ++k)
             for (int j = 0; j < 2; ++j)
                 for (int i = 0; i < 2; ++i) {
-                    const uint4 v = reinterpret_cast<const uint4*>(
-                        in + ((((long long)(2 * Z + k) * ny + 2 * Y + j) * nx) + 2 * X + i) * C)[c8];
                     float f[8];
-                    unpack8(v, f);
+                    unpack8(reinterpret_cast<const uint4*>(
+                                in + ((((long long)(2 * Z + k) * ny + 2 * Y + j) * nx) + 2 * X + i) * C)[c8],
+                            f);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) s[e] += f[e];
                 }
-        reinterpret_cast<uint4*>(out)[q] =
-            make_uint4(pack2(0.125f * s[0], 0.125f * s[1]), pack2(0.125f * s[2], 0.125f * s[3]),
-                       pack2(0.125f * s[4], 0.125f * s[5]), pack2(0.125f * s[6], 0.125f * s[7]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] *= 0.125f;
+        reinterpret_cast<uint4*>(out)[q] = pack8(s);
     }
 }
 
@@ -633,21 +645,20 @@ __global__ void k_up2_add(const bf16_t* __restrict__ low, const bf16_t* __restri
                           bf16_t* __restrict__ out, int nx, int ny, int nz, int C) {
     pdl_wait();
     pdl_release();
-    const int C8 = C / 8;
-    const long long n = (long long)nx * ny * nz * C8;
+    const int sh = __ffs(C) - 4, C8 = 1 << sh;
+    const long long n = (long long)nx * ny * nz << sh;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
          q += (long long)gridDim.x * blockDim.x) {
-        const int c8 = (int)(q % C8);
-        long long v = q / C8;
-        const int x = (int)(v % nx);
-        v /= nx;
-        const int y = (int)(v % ny), z = (int)(v / ny);
-        const long long P = (((long long)(z / 2) * (ny / 2) + y / 2) * (nx / 2) + x / 2) * C8 + c8;
+        const int c8 = (int)q & (C8 - 1);
+        const unsigned v = (unsigned)(q >> sh), r = v / nx;
+        const int x = v - r * nx, z = r / ny, y = r - z * ny;
+        const long long P = ((((long long)(z / 2) * (ny / 2) + y / 2) * (nx / 2) + x / 2) << sh) + c8;
         float a[8], b[8];
         unpack8(reinterpret_cast<const uint4*>(low)[P], a);
         unpack8(reinterpret_cast<const uint4*>(skip)[q], b);
-        reinterpret_cast<uint4*>(out)[q] = make_uint4(pack2(a[0] + b[0], a[1] + b[1]), pack2(a[2] + b[2], a[3] + b[3]),
-                                                      pack2(a[4] + b[4], a[5] + b[5]), pack2(a[6] + b[6], a[7] + b[7]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] += b[e];
+        reinterpret_cast<uint4*>(out)[q] = pack8(a);
     }
 }
 
@@ -657,21 +668,28 @@ __global__ void k_bwd_up_relu(const bf16_t* __restrict__ g, const bf16_t* __rest
                               bf16_t* __restrict__ out, int nx, int ny, int nz, int C) {
     pdl_wait();
     pdl_release();
-    const int hx = nx / 2, hy = ny / 2, hz = nz / 2;
-    const long long n = (long long)hx * hy * hz * C;
+    const int hx = nx / 2, hy = ny / 2, hz = nz / 2, sh = __ffs(C) - 4, C8 = 1 << sh;
+    const long long n = (long long)hx * hy * hz << sh;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
          q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        long long V = q / C;
-        const int X = (int)(V % hx);
-        V /= hx;
-        const int Y = (int)(V % hy), Z = (int)(V / hy);
-        float s = 0.f;
+        const int c8 = (int)q & (C8 - 1);
+        const unsigned V = (unsigned)(q >> sh), R = V / hx;
+        const int X = V - R * hx, Z = R / hy, Y = R - Z * hy;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, y[8];
         for (int k = 0; k < 2; ++k)
             for (int j = 0; j < 2; ++j)
-                for (int i = 0; i < 2; ++i)
-                    s += bf2f(g[((((long long)(2 * Z + k) * ny + 2 * Y + j) * nx) + 2 * X + i) * C + c]);
-        out[q] = bf2f(ylow[q]) > 0.f ? f2bf(s) : (bf16_t)0;
+                for (int i = 0; i < 2; ++i) {
+                    float f[8];
+                    unpack8(reinterpret_cast<const uint4*>(
+                                g + ((((long long)(2 * Z + k) * ny + 2 * Y + j) * nx) + 2 * X + i) * C)[c8],
+                            f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) s[e] += f[e];
+                }
+        unpack8(reinterpret_cast<const uint4*>(ylow)[q], y);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = y[e] > 0.f ? s[e] : 0.f;
+        reinterpret_cast<uint4*>(out)[q] = pack8(s);
     }
 }
 
@@ -681,17 +699,21 @@ __global__ void k_bwd_pool_skip_relu(const bf16_t* __restrict__ gpool, const bf1
                                      int ny, int nz, int C) {
     pdl_wait();
     pdl_release();
-    const long long n = (long long)nx * ny * nz * C;
+    const int sh = __ffs(C) - 4, C8 = 1 << sh;
+    const long long n = (long long)nx * ny * nz << sh;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
          q += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(q % C);
-        long long v = q / C;
-        const int x = (int)(v % nx);
-        v /= nx;
-        const int yy = (int)(v % ny), z = (int)(v / ny);
-        const long long P = (((long long)(z / 2) * (ny / 2) + yy / 2) * (nx / 2) + x / 2) * C + c;
-        const float s = 0.125f * bf2f(gpool[P]) + (gskip ? bf2f(gskip[q]) : 0.f);
-        out[q] = bf2f(y[q]) > 0.f ? f2bf(s) : (bf16_t)0;
+        const int c8 = (int)q & (C8 - 1);
+        const unsigned v = (unsigned)(q >> sh), r = v / nx;
+        const int x = v - r * nx, z = r / ny, yy = r - z * ny;
+        const long long P = ((((long long)(z / 2) * (ny / 2) + yy / 2) * (nx / 2) + x / 2) << sh) + c8;
+        float p[8], k[8], u[8];
+        unpack8(reinterpret_cast<const uint4*>(gpool)[P], p);
+        unpack8(reinterpret_cast<const uint4*>(gskip)[q], k);
+        unpack8(reinterpret_cast<const uint4*>(y)[q], u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) p[e] = u[e] > 0.f ? 0.125f * p[e] + k[e] : 0.f;
+        reinterpret_cast<uint4*>(out)[q] = pack8(p);
     }
 }
 
@@ -956,32 +978,32 @@ int backward(wpf_net* n, const bf16_t* x, cudaStream_t s) {
     if ((rc = wgrad(n, 6, n->s0, n->gout, false, s))) return rc;
     if ((rc = conv(n, 6, n->gout, n->L[6].wt16, 16, 16, false, n->gs0, nullptr, nullptr, true, s))) return rc;
     // layer 5
-    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[1] * 16), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[1] * 16 / 8), 256, 0, s,
                            n->gs0, n->y[5], n->gpre[5], X[0], Y[0], Z[0], 16));
     if ((rc = wgrad(n, 5, n->s1, n->gpre[5], true, s))) return rc;
     if ((rc = conv(n, 5, n->gpre[5], n->L[5].wt16, 16, 32, false, n->gs1, nullptr, nullptr, true, s))) return rc;
     // layer 4
-    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[2] * 32), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[2] * 32 / 8), 256, 0, s,
                            n->gs1, n->y[4], n->gpre[4], X[1], Y[1], Z[1], 32));
     if ((rc = wgrad(n, 4, n->s2, n->gpre[4], true, s))) return rc;
     if ((rc = conv(n, 4, n->gpre[4], n->L[4].wt16, 32, 64, false, n->gs2, nullptr, nullptr, true, s))) return rc;
     // layer 3
-    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[3] * 64), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_up_relu, ew_grid(n->nvox[3] * 64 / 8), 256, 0, s,
                            n->gs2, n->y[3], n->gpre[3], X[2], Y[2], Z[2], 64));
     if ((rc = wgrad(n, 3, n->p2, n->gpre[3], true, s))) return rc;
     if ((rc = conv(n, 3, n->gpre[3], n->L[3].wt16, 64, 64, false, n->gp2, nullptr, nullptr, true, s))) return rc;
     // layer 2
-    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[2] * 64), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[2] * 64 / 8), 256, 0, s,
                            n->gp2, n->gs2, n->y[2], n->gpre[2], X[2], Y[2], Z[2], 64));
     if ((rc = wgrad(n, 2, n->p1, n->gpre[2], true, s))) return rc;
     if ((rc = conv(n, 2, n->gpre[2], n->L[2].wt16, 64, 32, false, n->gp1, nullptr, nullptr, true, s))) return rc;
     // layer 1
-    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[1] * 32), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[1] * 32 / 8), 256, 0, s,
                            n->gp1, n->gs1, n->y[1], n->gpre[1], X[1], Y[1], Z[1], 32));
     if ((rc = wgrad(n, 1, n->p0, n->gpre[1], true, s))) return rc;
     if ((rc = conv(n, 1, n->gpre[1], n->L[1].wt16, 32, 16, false, n->gp0, nullptr, nullptr, true, s))) return rc;
     // layer 0
-    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[0] * 16), 256, 0, s,
+    WPF_CUDA(launch_behind(true, k_bwd_pool_skip_relu, ew_grid(n->nvox[0] * 16 / 8), 256, 0, s,
                            n->gp0, n->gs0, n->y[0], n->gpre[0], X[0], Y[0], Z[0], 16));
     if ((rc = wgrad(n, 0, x, n->gpre[0], true, s))) return rc;
     BiasArgs ba;
